@@ -6,8 +6,8 @@
 //   dk = b*(gamma*eb) + yb/gamma;  db = k*(gamma*eb);  dbeta = sum_k db + sum_v v*P
 //   dg = reverse chunk cumsum of  q*dq + k*b*(gamma*eb) - k*(yb/gamma)  (+ chunk-end term on the last row)
 // with Yc = k*zeta, Qc = q*alpha, Ec = b*k*alpha, alpha = exp2(g-c), zeta = 1/alpha and c the per-channel
-// mid-point of the chunk's cumulative gate; chunks whose gate span reaches 80 log2 units take an exact
-// pairwise path instead of the centered products.
+// mid-point of the chunk's cumulative gate; chunks whose gate span reaches VECTOR_SPAN_LIMIT (SCALAR_SPAN_LIMIT) log2
+// units take an exact pairwise path instead of the centered products.
 //
 // One kernel replaces, for all four families, the reference's residual-WY producer/consumer
 // (src/fast_delta_rule/kernels/kda_residual_tri_beta.py:9-73, kda_residual_local_beta_consumer.py:23-180),
@@ -22,7 +22,6 @@ namespace {
 constexpr int LD128 = 136;
 constexpr int LD64 = 72;
 constexpr int LDG = 132;  // pitch of the FP32 dg tile
-constexpr float SPAN_LIMIT = 80.f;
 
 struct ChunkParams {
   const bf16 *q, *k, *v, *bg, *wg, *Akk, *dO, *R, *h, *dh, *dR, *dRlo;
@@ -106,7 +105,7 @@ __device__ __forceinline__ void chunk_body(const ChunkParams& p, const int n, co
         hi = fmaxf(hi, x);
       }
       c = 0.5f * (lo + hi);
-      if (!(hi - lo < SPAN_LIMIT)) atomicOr(sFlag, 1);
+      if (!(hi - lo < VECTOR_SPAN_LIMIT)) atomicOr(sFlag, 1);
     } else if (GATE == GATE_SCALAR) {
       float lo = INFINITY, hi = -INFINITY;
       for (int r = 0; r < C; r++) {
@@ -114,7 +113,7 @@ __device__ __forceinline__ void chunk_body(const ChunkParams& p, const int n, co
         hi = fmaxf(hi, sGs[r]);
       }
       c = 0.5f * (lo + hi);
-      if (tid == 0 && !(hi - lo < SPAN_LIMIT)) atomicOr(sFlag, 1);
+      if (tid == 0 && !(hi - lo < SCALAR_SPAN_LIMIT)) atomicOr(sFlag, 1);
     }
     sCen[tid] = c;
   }

@@ -21,7 +21,7 @@
 //     into registers once; beta rows are double-buffered and fetched under a tensor-core wait;
 //   * dv and dg leave as tiles by bulk stores; per-token sums go through small per-warp arrays, per-channel
 //     sums through spare TMEM columns (no shared-memory atomics).
-// Chunks whose cumulative gate spans 80 or more log2 units are not processed here: their indices are appended
+// Chunks whose cumulative gate spans VECTOR_SPAN_LIMIT or more log2 units are not processed here: their indices are appended
 // to a list that the warp-MMA kernel (exact pairwise path) works off afterwards.
 #include <cstdio>
 #include "tc05.cuh"
@@ -29,8 +29,6 @@
 namespace rewy {
 namespace {
 using namespace tc;
-
-constexpr float SPAN_LIMIT = 80.f;
 
 // Division of a non-negative int below 2^31 by a divisor fixed at launch: quotient = umulhi(x, mul) >> shift.
 struct FastDiv {
@@ -411,7 +409,7 @@ chunk_adjoint_tc_kernel(const __grid_constant__ CUtensorMap tmAkk, const __grid_
       }
       if (GATE == GATE_VECTOR) {
         cen = 0.5f * (lo + hi);
-        wide = !(hi - lo < SPAN_LIMIT);
+        wide = !(hi - lo < VECTOR_SPAN_LIMIT);
       } else {
         // A scalar gate is the same for every channel, so its pairwise factor 2^(G_i - G_j), i >= j, is applied to the
         // 64x64 matrices themselves and no operand is scaled by a centred factor.  With a non-increasing cumulative
@@ -420,7 +418,7 @@ chunk_adjoint_tc_kernel(const __grid_constant__ CUtensorMap tmAkk, const __grid_
         bool rises = t0 > 0 && g[0] > sGs[t0 - 1];
 #pragma unroll
         for (int j = 1; j < HALF; j++) rises = rises || g[j] > g[j - 1];
-        wide = rises && !(hi - lo < SPAN_LIMIT);
+        wide = rises && !(hi - lo < SCALAR_SPAN_LIMIT);
       }
     }
     // the previous chunk's output tiles must have left shared memory before their regions are written again

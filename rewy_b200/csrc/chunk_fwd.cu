@@ -11,7 +11,7 @@
 // The two 64x64x128 products that build the A matrices use centred gate factors (alpha = 2^(G - c), zeta = 1/alpha with
 // c the per-channel mid-point of G over the chunk) and BF16 hi/lo operand pairs in three passes (about 16 mantissa
 // bits), accumulated in FP32 by warp-level MMA (operands by ldmatrix); scalar gates apply their pairwise factor 2^(G_i - G_j) to the exact
-// q k^T and k k^T products instead.  A chunk whose cumulative gate spans 80 log2 units or more in some channel does not
+// q k^T and k k^T products instead.  A chunk whose cumulative gate spans VECTOR_SPAN_LIMIT log2 units or more in some channel does not
 // use centred factors (they would leave the FP32 range): its two matrices are summed pair by pair on the CUDA cores,
 // sum_k q_ik k_jk 2^(G_ik - G_jk), like the exact pairwise path of the backward.  The unit lower-triangular inverse is
 // plain FP32 forward substitution, one thread per column with the column held in registers.
@@ -26,7 +26,6 @@ constexpr int LD128 = 136;  // padded pitch of a 128-wide BF16 tile
 constexpr int LD64 = 72;    // padded pitch of a 64-wide BF16 tile
 constexpr int LDL = 68;     // padded pitch of the FP32 64x64 matrix (rows stay 16-byte aligned)
 constexpr int LDG = 132;    // padded pitch of the FP32 gate tile of a wide-span chunk
-constexpr float FWD_SPAN_LIMIT = 80.f;
 
 struct FwdLocalParams {
   const bf16 *q, *k, *v, *bg, *wg;
@@ -128,7 +127,7 @@ __global__ void __launch_bounds__(256, 3) chunk_fwd_local_kernel(const FwdLocalP
     }
     sGl[tid] = last;
     sCen[tid] = 0.5f * (lo + hi);
-    wide_here = !(hi - lo < FWD_SPAN_LIMIT);
+    wide_here = !(hi - lo < VECTOR_SPAN_LIMIT);
   }
   // wide gate span somewhere in the chunk: no centred factors, exact pairwise sums instead (vector gate only)
   const bool wide = __syncthreads_or(wide_here ? 1 : 0) != 0;
@@ -147,7 +146,7 @@ __global__ void __launch_bounds__(256, 3) chunk_fwd_local_kernel(const FwdLocalP
       load_gate8(p.g + go, gg);
 #pragma unroll
       for (int j = 0; j < 8; j++) {
-        const float al = ex2(gg[j] - sCen[c + j]);  // |exponent| < 40: no flush
+        const float al = ex2(gg[j] - sCen[c + j]);  // |exponent| < 80: no flush
         qc[j] = qq[j] * al;
         yc[j] = kk[j] * rcp(al);
       }
