@@ -10,22 +10,11 @@
 //   epilogue    thread (value channel, token half) stores dR as BF16 hi/lo to global and (dR/scale) hi/lo tiles
 //   MMA 2       S'[k,v] += sum_i qg[i,k] dO[i,v] - sum_i w[i,k] (dR/scale)[i,v]                 M=128 N=128
 // Every operand that comes from global memory is used exactly as TMA lands it (MN-major or K-major).
-#include "tc05.cuh"
+#include "state_scan_tc.cuh"
 
 namespace rewy {
 namespace {
-using namespace tc;
-
-struct ScanParams {
-  const float *g, *dht;
-  bf16 *dR, *dRlo;
-  float* dh0;
-  int* err;
-  int T, H, NT;
-  int svf;  // initial / final state tensors (dht, dh0) are stored value-first: [B,H,V,K]
-  const int* cu;  // packed sequences: device int32 [sequences + 1] token offsets (multiples of 64), or nullptr
-  float scale;
-};
+using namespace scan;
 
 // Shared-memory plan, byte offsets from a 1024-byte aligned base.  The 64 KB region X is time-shared inside a chunk:
 // first the dh hi/lo tiles (operands of the dR product), then - once that product is done - qg, w and the
@@ -50,52 +39,6 @@ static_assert(2 * (SS::TOTAL + 2048) <= 233472, "two reverse-scan CTAs must fit 
 enum { B_L1 = 0, B_DO, B_L2, B_DR, B_S };
 constexpr uint32_t TM_S = 0, TM_DR = 128;
 constexpr int TPB = 256;
-
-__device__ __forceinline__ void tmem_ld16f(uint32_t taddr, float (&r)[16]) {
-  uint32_t u[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]),
-        "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
-      : "r"(taddr)
-      : "memory");
-#pragma unroll
-  for (int i = 0; i < 16; i++) r[i] = __uint_as_float(u[i]);
-}
-__device__ __forceinline__ void tmem_st16f(uint32_t taddr, const float (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
-      "r"(__float_as_uint(r[0])), "r"(__float_as_uint(r[1])), "r"(__float_as_uint(r[2])), "r"(__float_as_uint(r[3])),
-      "r"(__float_as_uint(r[4])), "r"(__float_as_uint(r[5])), "r"(__float_as_uint(r[6])), "r"(__float_as_uint(r[7])),
-      "r"(__float_as_uint(r[8])), "r"(__float_as_uint(r[9])), "r"(__float_as_uint(r[10])), "r"(__float_as_uint(r[11])),
-      "r"(__float_as_uint(r[12])), "r"(__float_as_uint(r[13])), "r"(__float_as_uint(r[14])), "r"(__float_as_uint(r[15]))
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// shared -> global tile store through a tensor map (bulk async group of the issuing thread)
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, int c0, int c1, const void* src) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
-                   reinterpret_cast<uint64_t>(m)),
-               "r"(smem_u32(src)), "r"(c0), "r"(c1)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-
-__device__ __forceinline__ void split8s(const float (&x)[8], uint4& hi, uint4& lo) {
-  uint32_t h[4], l[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    __nv_bfloat162 hh = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
-    float2 hf = __bfloat1622float2(hh);
-    h[i] = *reinterpret_cast<uint32_t*>(&hh);
-    l[i] = pack_bf16(x[2 * i] - hf.x, x[2 * i + 1] - hf.y);
-  }
-  hi = make_uint4(h[0], h[1], h[2], h[3]);
-  lo = make_uint4(l[0], l[1], l[2], l[3]);
-}
 
 template <int GATE>
 __global__ void __launch_bounds__(TPB, 2)
@@ -261,21 +204,20 @@ bwd_scan_tc_kernel(const __grid_constant__ CUtensorMap tmKg, const __grid_consta
         for (int pn = 0; pn < 2; pn++) tma_store_2d(&tmDH, 64 * pn, hrow0, sm + SS::DHHI + pn * 16384);
         bulk_commit();
       }
+      // dO^T Aqk first, as in state_scan_split.cu: a sequence's result does not depend on how many run with it
       wait(B_L1, 2);
+      wait(B_DO, 3);  // requested at the top of the chunk: its latency hides behind the work on the state row
       if (alive) {
         tc_fence_after_sync();
+        for (int ks = 0; ks < 4; ks++)
+          mma_f16(tb + TM_DR, smem_desc(sb + SS::DO0 + ks * 2048, 8192, 1024),
+                  smem_desc(sb + SS::AQK + ks * 2048, 8192, 1024), ID_DR_B, ks > 0);
         for (int pass = 0; pass < 2; pass++) {
           const uint32_t a = sb + (pass == 0 ? SS::DHHI : SS::DHLO);
           for (int ks = 0; ks < 8; ks++)
             mma_f16(tb + TM_DR, smem_desc(a + ks * 2048, 16384, 1024),
-                    smem_desc(sb + SS::KG + (ks >> 2) * 8192 + (ks & 3) * 32, 16, 1024), ID_DR_A, pass > 0 || ks > 0);
+                    smem_desc(sb + SS::KG + (ks >> 2) * 8192 + (ks & 3) * 32, 16, 1024), ID_DR_A, true);
         }
-      }
-      wait(B_DO, 3);  // dO was requested at the top of the chunk: its latency hides behind the products above
-      if (alive) {
-        for (int ks = 0; ks < 4; ks++)
-          mma_f16(tb + TM_DR, smem_desc(sb + SS::DO0 + ks * 2048, 8192, 1024),
-                  smem_desc(sb + SS::AQK + ks * 2048, 8192, 1024), ID_DR_B, true);
         mma_commit(&bars[B_DR]);
       }
     } else {
@@ -374,15 +316,6 @@ bwd_scan_tc_kernel(const __grid_constant__ CUtensorMap tmKg, const __grid_consta
 // Replaces FLA chunk_gated_delta_rule_fwd_h (src/fast_delta_rule/backends/backward.py:117-118).  Same layout
 // tricks as the reverse scan; operands are single BF16 (h and v_new are exactly the tensors that get saved), so it
 // needs 97 KB of shared memory and 192 TMEM columns and two CTAs share an SM.
-struct FwdParams {
-  const float *g, *h0;
-  float* final_state;  // optional: state after the last chunk, FP32 [B,H,K,V] ([B,H,V,K] when svf)
-  bf16* v_new;
-  int* err;
-  int T, H, NT;
-  int svf;  // h0 is stored value-first: [B,H,V,K]
-  const int* cu;  // packed sequences: device int32 [sequences + 1] token offsets (multiples of 64), or nullptr
-};
 struct FS {
   static constexpr uint32_t W = 0;                // [64 i][128 k] two panels   16 KB
   static constexpr uint32_t KG = W + 16384;       // [64 i][128 k]              16 KB
@@ -660,6 +593,7 @@ cudaError_t launch_bwd_scan_tc(const RewyBwdArgs& a, const RewyStageBuffers& s, 
   p.g = a.g; p.dht = a.dht; p.dR = (bf16*)s.dR; p.dRlo = (bf16*)s.dR_lo; p.dh0 = a.dh0; p.err = err;
   p.T = T; p.H = H; p.NT = NT; p.svf = a.state_v_first; p.cu = a.cu_seqlens; p.scale = a.scale;
   const int seqs = a.cu_seqlens != nullptr ? a.num_seqs : B;  // one CTA per (sequence, head)
+  if (seqs * H <= SPLIT_MAX_PAIRS) return launch_bwd_scan_split(gate_mode_of(a.family), tm, p, seqs * H, st);
   switch (gate_mode_of(a.family)) {
     case GATE_NONE: return run<GATE_NONE>(tm, p, seqs * H, st);
     case GATE_SCALAR: return run<GATE_SCALAR>(tm, p, seqs * H, st);
@@ -682,6 +616,7 @@ cudaError_t launch_fwd_scan_tc(const RewyBwdArgs& a, const RewyStageBuffers& s, 
   p.g = a.g; p.h0 = a.h0; p.final_state = final_state; p.v_new = (bf16*)s.v_new; p.err = err; p.T = T; p.H = H; p.NT = NT; p.svf = a.state_v_first;
   p.cu = a.cu_seqlens;
   const int seqs = a.cu_seqlens != nullptr ? a.num_seqs : B;  // one CTA per (sequence, head)
+  if (seqs * H <= SPLIT_MAX_PAIRS) return launch_fwd_scan_split(gate_mode_of(a.family), tm, p, seqs * H, st);
   switch (gate_mode_of(a.family)) {
     case GATE_NONE: return run_fwd<GATE_NONE>(tm, p, seqs * H, st);
     case GATE_SCALAR: return run_fwd<GATE_SCALAR>(tm, p, seqs * H, st);

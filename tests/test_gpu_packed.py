@@ -62,6 +62,29 @@ def test_packed_batch_equals_its_sequences_run_one_at_a_time(op, saved):
         at += T
 
 
+@pytest.mark.parametrize("op,saved", [("kda", True), ("gdn2", False), ("gdn", False), ("delta", False)])
+def test_many_packed_pairs_give_what_few_give(op, saved):
+    """160 (sequence, head) pairs go to the whole-state scans, the 32 of a single sequence to the scans split by value
+    channels (limit: 148 pairs); both sum in the same order, so the results are equal to the last bit.  One, two and three
+    chunks."""
+    H, lengths = 32, (64, 192, 128, 64, 128)
+    seqs = [make_inputs(op, 1, T, H, seed=70 + i, device=DEV, gate_scale=0.1, gate="softplus") for i, T in enumerate(lengths)]
+    packed = {n: torch.cat([s[n] for s in seqs], 1) for n in ARGS[op]}
+    state = lambda n: torch.cat([s[n] for s in seqs], 0)
+    h0, dht, do = state("initial_state"), state("dht"), torch.cat([s["do"] for s in seqs], 1)
+    cu = torch.cat([torch.zeros(1, dtype=torch.int64), torch.tensor(lengths).cumsum(0)]).to(DEV)
+    o, fin, grads = _run(op, packed, h0, do, dht, saved, cu)
+    at = 0
+    for row, s in enumerate(seqs):
+        T = s["q"].shape[1]
+        o1, fin1, g1 = _run(op, {n: s[n] for n in ARGS[op]}, s["initial_state"], s["do"], s["dht"], saved)
+        assert torch.equal(o[:, at:at + T], o1) and torch.equal(fin[row:row + 1], fin1), (op, row)
+        for n in ARGS[op]:
+            assert torch.equal(grads[n][:, at:at + T], g1[n]), (op, row, n)
+        assert torch.equal(grads["initial_state"][row:row + 1], g1["initial_state"]), (op, row)
+        at += T
+
+
 def test_offsets_that_do_not_match_the_token_count_are_refused_and_the_kernels_check_lengths():
     """The operators refuse offsets that do not add up on the host (lengths that are not multiples of 64 are padded
     there, tests/test_gpu_envelope.py); the scan kernels, given such offsets directly, record the length in the status
