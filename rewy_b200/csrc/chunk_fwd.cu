@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(256, 3) chunk_fwd_local_kernel(const FwdLocalP
       load_gate8(p.g + go, gg);
 #pragma unroll
       for (int j = 0; j < 8; j++) {
-        const float al = ex2(gg[j] - sCen[c + j]);  // |exponent| < 80: no flush
+        const float al = ex2(gg[j] - sCen[c + j]);  // |exponent| < 100: no flush
         qc[j] = qq[j] * al;
         yc[j] = kk[j] * rcp(al);
       }

@@ -17,12 +17,13 @@ using bf16 = __nv_bfloat16;
 
 // Largest span (max - min over the 64 tokens of a chunk, log2 units) of a per-channel cumulative gate that the centred
 // factors 2^(G - c), 2^(c - G) take: a chunk that reaches it is summed pair by pair on the CUDA cores, some thirty times
-// as slow.  The factors stay inside 2^-80 .. 2^80, so an operand's BF16 hi and lo parts stay normal numbers for every
-// |q|, |k| above 2^-30 and a sum over the kept (causal) entries stays in FP32 range; entries above the diagonal may
-// overflow and are selected away, never multiplied.  A layer with decay rates up to 16 and time steps up to 0.1 spans up
-// to about 150: at a limit of 80 the pairwise path took 71 % of such a layer's chunks and, at B=2 T=4096 H=16, 3.65 ms of
-// its backward and 0.55 ms of its forward.
-constexpr float VECTOR_SPAN_LIMIT = 160.f;
+// as slow.  The factors stay inside 2^-100 .. 2^100.  Below 2^-126 an operand's BF16 lo part is lost: that changes a sum
+// by 2^-126 times the other factor, at most 2^-26 of an entry of size 1, while the hi/lo products carry 2^-16; a sum over
+// the kept (causal) entries stays in FP32 range up to 2^27 times an entry of size 1; entries above the diagonal may
+// overflow and are selected away, never multiplied.  A layer with decay rates up to 16 and time steps up to 0.1 averages
+// up to 165 in its fastest channel.  At B=2 T=4096 H=16 with such a gate: a limit of 80 sent 71 % of the chunks to the
+// pairwise sums (3.65 ms of the backward, 0.55 ms of the forward), 160 a few (0.41 ms and 0.10 ms), 200 none.
+constexpr float VECTOR_SPAN_LIMIT = 200.f;
 // A scalar gate needs no centred factors unless it rises (its pairwise factor is applied to the 64x64 matrices): limit of
 // the chunks that do.
 constexpr float SCALAR_SPAN_LIMIT = 80.f;
