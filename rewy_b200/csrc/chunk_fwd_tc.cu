@@ -1,20 +1,23 @@
 // Chunk-local forward stage on the Blackwell tensor cores: Akk, Aqk, w, u, qg, kg of every chunk (definitions and the
 // reference functions it replaces: chunk_fwd.cu).
 //
-// Persistent, two CTAs per SM; per chunk:
+// Persistent, two CTAs of 256 threads per SM; per chunk:
 //   * TMA brings q and k (one 128-row operand [q ; k]), g, later v;
 //   * vector gate: thread (row of [q ; k], 64 channels) turns its row into Qc = q alpha or Ec = b k alpha, BF16 hi and
 //     lo, written straight into TENSOR MEMORY as the A operand; the q rows also write Yc = k / alpha (hi, lo) as the
-//     shared-memory B operand and qg in place of q, the k rows keep E = b k gamma and kg in registers until the
-//     inputs are dead.  One pass over the inputs and four MUFU results per element make everything
-//     (gamma = alpha 2^c, applied as two factors 2^(c/2) so that no intermediate leaves the FP32 range);
+//     shared-memory B operand;
 //   * [Qc ; Ec] Yc^T is ONE M=128 product in three hi/lo passes (scalar gate / none: [q ; k] k^T, exact, one pass, on
-//     the tiles as they landed): lanes 0..63 give Aqk, lanes 64..127 the matrix to invert;
-//   * (I + L)^-1 in FP32 by blocks 16 -> 32 -> 64 with all 256 threads: X21 = -X22 (L21 X11);
+//     the tiles as they landed): lanes 0..63 give Aqk, lanes 64..127 the matrix to invert.  While it runs qg and kg
+//     leave in 16-byte pieces and E = b k gamma takes the place of k;
+//   * (I + L)^-1 in FP32 by blocks 16 -> 32 -> 64 with all threads: X21 = -X22 (L21 X11);
 //   * w = Akk E and u = Akk Z with Akk stored twice (M=128), so that lanes 0..63 finish w and lanes 64..127 u.
 // A chunk whose gate spans VECTOR_SPAN_LIMIT uses no centred factors: its two matrices are summed pair by pair here.
-// Measured, against the warp-MMA kernel this replaces (three passes over the inputs, inverse by 64 threads): KDA B=1
-// T=8192 H=32 336 -> 251 us, GDN B=2 T=4096 H=32 202 -> 150 us, GDN2 B=2 T=2048 H=8 68 -> 45 us.
+// The loops are kept rolled (two deep): a chunk's code runs once per chunk, and with everything unrolled the warps waited
+// for instructions more than for anything else (1.9 of 10 cycles per issued instruction, more than for memory).
+// Measured, against the warp-MMA kernel before it (three passes over the inputs, inverse by 64 threads): KDA B=1 T=8192
+// H=32 336 -> 217 us, GDN B=2 T=4096 H=32 202 -> 148 us, GDN2 B=2 T=2048 H=8 68 -> 41 us.  Unrolled: 251, 150, 45; with
+// 512 threads per CTA: 237, 167, 41 (more instructions per result in the inverse).  Bound by instruction issue of the
+// operand pass and by the inverse's chain (5000 of 16000 cycles of a chunk without a vector gate).
 #include "tc05.cuh"
 
 namespace rewy {
@@ -22,13 +25,14 @@ namespace {
 using namespace tc;
 
 constexpr int TPB = 256;
+constexpr int NG = TPB / 128;  // column groups: a thread has 1/NG of its TMEM lane's columns
 constexpr int LDL = 68;  // pitch of the FP32 matrix (16-byte rows, conflict-free by rows and by columns of four)
 constexpr unsigned long long DRAIN_NS = 20ull * 1000 * 1000;
 
 struct LocalParams {
   const float *g, *beta;
   const bf16 *bg, *wg;
-  bf16 *Akk, *Aqk;
+  bf16 *Akk, *Aqk, *qg, *kg;
   int* err;
   int T, H, NT, total_chunks;
   int write_qk;  // 0: no gate and the caller's qg, kg are q and k themselves
@@ -40,27 +44,39 @@ struct LS {
   static constexpr uint32_t QK = 0;                // [q ; k] panel 0 (q 8 KB, k 8 KB), panel 1           32 KB
   static constexpr uint32_t KT = QK + 8192;        // k panels, 16 KB apart; become E, then w
   static constexpr uint32_t G = QK + 32768;        // vector gate: 4 panels [64 t][32 k] FP32              32 KB
-  static constexpr uint32_t KG = G;                // kg panels over the dead gate tile                    16 KB
-  static constexpr uint32_t L = G + 16384;         // FP32 [64][68]: L, then (I + L)^-1                    17 KB
-  static constexpr uint32_t Y = G + 33792;         // Yc hi panels, lo panels                              32 KB
-  static constexpr uint32_t V = Y;                 // v panels; become Z, then u                           16 KB
-  static constexpr uint32_t AK = Y + 16384;        // Akk twice: 128 rows K-major                          16 KB
-  static constexpr uint32_t CEN = Y + 32768;       // float[128] centre of the gate
-  static constexpr uint32_t E2H = CEN + 512;       // float[128] 2^(centre / 2)
-  static constexpr uint32_t GL = E2H + 512;        // float[128] last gate row
-  static constexpr uint32_t MM = GL + 512;         // float[2][2][128] min / max of the row halves
-  static constexpr uint32_t BETA = MM + 2048;      // float[64]
+  static constexpr uint32_t Y = G + 32768;         // Yc hi panels, lo panels                              32 KB
+  static constexpr uint32_t L = Y;                 // over Yc: FP32 [64][68]: L, then (I + L)^-1           17 KB
+  static constexpr uint32_t AK = L + 64 * LDL * 4; //          Akk twice: 128 rows K-major                 16 KB
+  static constexpr uint32_t CEN = AK + 16384;      // float[128] centre of the gate
+  static constexpr uint32_t GL = CEN + 512;        // float[128] last gate row
+  static constexpr uint32_t MM = GL + 512;         // float[NG][2][128] min / max of the row groups
+  static constexpr uint32_t BETA = MM + NG * 1024; // float[64]
   static constexpr uint32_t GS = BETA + 256;       // float[64] scalar gate rows
   static constexpr uint32_t BARS = GS + 256;
   static constexpr uint32_t TMEM = BARS + 64;
   static constexpr uint32_t TOTAL = TMEM + 64;
 };
-static_assert(LS::L + 64 * LDL * 4 == LS::Y && LS::Y % 1024 == 0, "the FP32 matrix ends where Yc begins");
+// v panels (then Z, then u): over q with a vector gate (pitch 16 KB), else where the gate tile would be (8 KB)
+template <int GATE> struct VPlace {
+  static constexpr uint32_t AT = GATE == GATE_VECTOR ? LS::QK : LS::G, PITCH = GATE == GATE_VECTOR ? 16384 : 8192;
+};
+static_assert(LS::AK % 1024 == 0 && LS::AK + 16384 >= LS::Y + 32768, "operand tiles on swizzle atoms, behind Yc");
 static_assert(2 * (LS::TOTAL + 1024) <= 233472, "two forward chunk CTAs must fit one SM");
 // TMEM columns: A operand hi / lo and the accumulator of the first product; then w and u
 constexpr uint32_t TM_A = 0, TM_D = 128, TM_W = 0, TM_U = 128;
-enum { LB_QG = 0, LB_K, LB_V, LB_D, LB_WU, LB_COUNT };
+enum { LB_G = 0, LB_QK, LB_V, LB_D, LB_WU, LB_COUNT };
 
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&r)[16]) {
+  uint32_t u[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]),
+        "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
+      : "r"(taddr)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 16; i++) r[i] = __uint_as_float(u[i]);
+}
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -139,7 +155,7 @@ __device__ __forceinline__ void invert_unit_lower(float* sL, int tid) {
     float* base = sL + 32 * p * (LDL + 1);         // X11; X22 16 further along the diagonal, L21 below X11
     float* tmp = sL + (16 * p) * LDL + 32;         // scratch 16 x 16
     float a0 = 0.f, a1 = 0.f;
-#pragma unroll
+#pragma unroll 2
     for (int k = 0; k < 16; k += 4) {
       const float4 l4 = *reinterpret_cast<const float4*>(base + (16 + i) * LDL + k);
       const float l[4] = {l4.x, l4.y, l4.z, l4.w};
@@ -153,7 +169,7 @@ __device__ __forceinline__ void invert_unit_lower(float* sL, int tid) {
     *reinterpret_cast<float2*>(tmp + i * LDL + c) = make_float2(a0, a1);
     __syncthreads();
     a0 = a1 = 0.f;
-#pragma unroll
+#pragma unroll 2
     for (int k = 0; k < 16; k += 4) {
       const float4 l4 = *reinterpret_cast<const float4*>(base + (16 + i) * LDL + 16 + k);
       const float l[4] = {l4.x, l4.y, l4.z, l4.w};
@@ -171,7 +187,7 @@ __device__ __forceinline__ void invert_unit_lower(float* sL, int tid) {
     const int i = tid >> 3, c = (tid & 7) * 4;
     float* tmp = sL + 32;  // rows 0..31, columns 32..63
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
+#pragma unroll 2
     for (int k = 0; k < 32; k += 4) {
       const float4 l4 = *reinterpret_cast<const float4*>(sL + (32 + i) * LDL + k);
       const float l[4] = {l4.x, l4.y, l4.z, l4.w};
@@ -184,7 +200,7 @@ __device__ __forceinline__ void invert_unit_lower(float* sL, int tid) {
     *reinterpret_cast<float4*>(tmp + i * LDL + c) = a;
     __syncthreads();
     a = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
+#pragma unroll 2
     for (int k = 0; k < 32; k += 4) {
       const float4 l4 = *reinterpret_cast<const float4*>(sL + (32 + i) * LDL + 32 + k);
       const float l[4] = {l4.x, l4.y, l4.z, l4.w};
@@ -203,13 +219,12 @@ template <int GATE, bool VB>
 __global__ void __launch_bounds__(TPB, 2)
 chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmG,
-                    const __grid_constant__ CUtensorMap tmQg, const __grid_constant__ CUtensorMap tmKg,
                     const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmU, const LocalParams p) {
   extern __shared__ __align__(1024) unsigned char sm[];
   constexpr bool VEC = GATE == GATE_VECTOR;
+  constexpr uint32_t VT = VPlace<GATE>::AT, VP = VPlace<GATE>::PITCH;
   float* sL = reinterpret_cast<float*>(sm + LS::L);
   float* sCen = reinterpret_cast<float*>(sm + LS::CEN);
-  float* sE2 = reinterpret_cast<float*>(sm + LS::E2H);
   float* sGl = reinterpret_cast<float*>(sm + LS::GL);
   float* sMM = reinterpret_cast<float*>(sm + LS::MM);
   float* sBeta = reinterpret_cast<float*>(sm + LS::BETA);
@@ -224,14 +239,13 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (tid == 0) atomicCAS(p.err, 0, 40);
     return;
   }
-  // thread = (row t of q or k, 64 channels): TMEM lanes 0..63 are rows of q, 64..127 rows of k
+  // thread = (row t of q or k, a quarter of the columns): TMEM lanes 0..63 are rows of q, 64..127 rows of k
   const int t = (warp & 1) * 32 + lane, krow = (warp >> 1) & 1, wg = warp >> 2;
 
   if (tid == 0) {
     for (int i = 0; i < LB_COUNT; i++) mbar_init(&bars[i], 1);
     fence_barrier_init();
-    prefetch_tmap(&tmQ); prefetch_tmap(&tmK); prefetch_tmap(&tmV); prefetch_tmap(&tmQg); prefetch_tmap(&tmKg);
-    prefetch_tmap(&tmW); prefetch_tmap(&tmU);
+    prefetch_tmap(&tmQ); prefetch_tmap(&tmK); prefetch_tmap(&tmV); prefetch_tmap(&tmW); prefetch_tmap(&tmU);
     if (VEC) prefetch_tmap(&tmG);
   }
   if (warp == 0) {
@@ -247,7 +261,7 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint32_t ph = 0;
   bool alive = true;
   auto wait = [&](int b, int code) {
-    if (alive) alive = mbar_wait(&bars[b], ph, p.err, code);  // every barrier completes once per chunk
+    if (alive) alive = mbar_wait(&bars[b], ph, p.err, code);  // every barrier in use completes once per chunk
   };
   auto dl = [&](uint32_t off, uint32_t lbo) { return desc_lo(sb + off, lbo); };
   struct Where { int h, row0; };
@@ -255,21 +269,23 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const int bn = chunk / H, h = chunk - bn * H, b = bn / NT, n = bn - b * NT;  // head fastest
     return Where{h, b * T + n * C};
   };
-  auto load_qg = [&](int chunk) {  // q and the gate
+  auto load_g = [&](int chunk) {
     const Where w = where(chunk);
-    mbar_expect_tx(&bars[LB_QG], 16384 + (VEC ? 32768 : 0));
-    for (int pn = 0; pn < 2; pn++) tma_load_2d(sm + LS::QK + pn * 16384, &tmQ, w.h * 128 + 64 * pn, w.row0, &bars[LB_QG]);
-    if (VEC) tma_load_3d(sm + LS::G, &tmG, w.h * 128, w.row0, 0, &bars[LB_QG]);
+    mbar_expect_tx(&bars[LB_G], 32768);
+    tma_load_3d(sm + LS::G, &tmG, w.h * 128, w.row0, 0, &bars[LB_G]);
   };
-  auto load_k = [&](int chunk) {
+  auto load_qk = [&](int chunk) {
     const Where w = where(chunk);
-    mbar_expect_tx(&bars[LB_K], 16384);
-    for (int pn = 0; pn < 2; pn++) tma_load_2d(sm + LS::KT + pn * 16384, &tmK, w.h * 128 + 64 * pn, w.row0, &bars[LB_K]);
+    mbar_expect_tx(&bars[LB_QK], 32768);
+    for (int pn = 0; pn < 2; pn++) {
+      tma_load_2d(sm + LS::QK + pn * 16384, &tmQ, w.h * 128 + 64 * pn, w.row0, &bars[LB_QK]);
+      tma_load_2d(sm + LS::KT + pn * 16384, &tmK, w.h * 128 + 64 * pn, w.row0, &bars[LB_QK]);
+    }
   };
   auto load_v = [&](int chunk) {
     const Where w = where(chunk);
     mbar_expect_tx(&bars[LB_V], 16384);
-    for (int pn = 0; pn < 2; pn++) tma_load_2d(sm + LS::V + pn * 8192, &tmV, w.h * 128 + 64 * pn, w.row0, &bars[LB_V]);
+    for (int pn = 0; pn < 2; pn++) tma_load_2d(sm + VT + pn * VP, &tmV, w.h * 128 + 64 * pn, w.row0, &bars[LB_V]);
   };
   float next_row = 0.f;  // beta (threads 0..63) or the scalar gate (64..127) of the next chunk's rows
   auto fetch_rows = [&](int chunk) {
@@ -284,9 +300,9 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   constexpr uint32_t ID_WU = instr_desc(FMT_BF16, 128, 128, false, true);  // A K-major (Akk), B MN-major (E / Z)
 
   if (leader && (int)blockIdx.x < p.total_chunks) {
-    load_qg(blockIdx.x);
-    load_k(blockIdx.x);
-    if (!VEC) load_v(blockIdx.x);
+    load_qk(blockIdx.x);
+    if (VEC) load_g(blockIdx.x);
+    else load_v(blockIdx.x);
   }
   __syncwarp();
   fetch_rows(blockIdx.x);
@@ -298,112 +314,84 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (!VB && tid < C) sBeta[tid] = next_row;
     if (GATE == GATE_SCALAR && tid >= C && tid < 2 * C) sGs[tid - C] = next_row;
     fetch_rows(next);
-    if (leader && next < p.total_chunks) {  // the next chunk's inputs into L2
-      const Where w = where(next);
-      for (int pn = 0; pn < 2; pn++) {
-        prefetch_2d(&tmK, w.h * 128 + 64 * pn, w.row0);
-        prefetch_2d(&tmV, w.h * 128 + 64 * pn, w.row0);
+    if (leader) {  // what is requested late goes to L2 now: this chunk's v, the next one's q and k
+      if (VEC)
+        for (int pn = 0; pn < 2; pn++) prefetch_2d(&tmV, h * 128 + 64 * pn, row0);
+      if (next < p.total_chunks) {
+        const Where w = where(next);
+        for (int pn = 0; pn < 2; pn++) {
+          prefetch_2d(&tmQ, w.h * 128 + 64 * pn, w.row0);
+          prefetch_2d(&tmK, w.h * 128 + 64 * pn, w.row0);
+          if (!VEC) prefetch_2d(&tmV, w.h * 128 + 64 * pn, w.row0);
+        }
       }
     }
     __syncwarp();
     bool wide = false;
-    uint4 epk[VEC ? 8 : 1], kpk[VEC ? 8 : 1];  // E and kg of a k row, until the inputs are dead
 
     if (VEC) {
       // ---- centre of the gate per channel ---------------------------------------------------------------------
-      wait(LB_QG, 41);
+      wait(LB_G, 41);
       {
-        const int ch = tid & 127, hf = tid >> 7;
+        const int ch = tid & 127, rg = tid >> 7;
         const unsigned char* gp = sm + LS::G + (ch >> 5) * 8192 + (ch & 3) * 4;
         float lo = INFINITY, hi = -INFINITY, last = 0.f;
-#pragma unroll 16
-        for (int r = 0; r < 32; r++) {
-          last = *reinterpret_cast<const float*>(gp + swz(32 * hf + r, (ch & 31) >> 2));
+#pragma unroll 8
+        for (int r = 0; r < C / NG; r++) {
+          last = *reinterpret_cast<const float*>(gp + swz(C / NG * rg + r, (ch & 31) >> 2));
           lo = fminf(lo, last);
           hi = fmaxf(hi, last);
         }
-        // (a NaN gate compares false everywhere and fminf / fmaxf drop it: it reaches the results through alpha)
-        sMM[hf * 256 + ch] = lo;
-        sMM[hf * 256 + 128 + ch] = hi;
-        if (hf == 1) sGl[ch] = last;
+        sMM[rg * 256 + ch] = lo;
+        sMM[rg * 256 + 128 + ch] = hi;
+        if (rg == NG - 1) sGl[ch] = last;
       }
       __syncthreads();
       if (tid < 128) {
-        const float lo = fminf(sMM[tid], sMM[256 + tid]), hi = fmaxf(sMM[128 + tid], sMM[384 + tid]);
-        const float c = 0.5f * (lo + hi);
-        sCen[tid] = c;
-        sE2[tid] = ex2(0.5f * c);
+        float lo = sMM[tid], hi = sMM[128 + tid];
+#pragma unroll
+        for (int rg = 1; rg < NG; rg++) {
+          lo = fminf(lo, sMM[rg * 256 + tid]);
+          hi = fmaxf(hi, sMM[rg * 256 + 128 + tid]);
+        }
+        sCen[tid] = 0.5f * (lo + hi);
         wide = !(hi - lo < VECTOR_SPAN_LIMIT);
       }
       wide = __syncthreads_or(wide ? 1 : 0) != 0;
-      wait(LB_K, 42);
-      // ---- operands -------------------------------------------------------------------------------------------
+      wait(LB_QK, 42);
+      // ---- operands of the first product ----------------------------------------------------------------------
       if (alive) {
         const float bs = VB ? 0.f : sBeta[t];
-#pragma unroll
-        for (int c8 = 0; c8 < 8; c8++) {
-          const int c = wg * 64 + c8 * 8;
-          const uint32_t off = swz(t, c8);
+#pragma unroll 2
+        for (int c8 = 0; c8 < 16 / NG; c8++) {
+          const int c = wg * (128 / NG) + c8 * 8;
+          const uint32_t pn = c >> 6, off = swz(t, (c & 63) >> 3);
           const unsigned char* gp = sm + LS::G + (c >> 5) * 8192;
-          float gg[8], kk[8], cen[8], e2[8];
-          load8(gp + swz(t, (c8 & 3) * 2), gp + swz(t, (c8 & 3) * 2 + 1), gg);
-          unpack8(*reinterpret_cast<const uint4*>(sm + LS::KT + wg * 16384 + off), kk);
-          load8(sm + LS::CEN + c * 4, sm + LS::CEN + c * 4 + 16, cen);
-          load8(sm + LS::E2H + c * 4, sm + LS::E2H + c * 4 + 16, e2);
+          float al[8], kk[8], x[8];
           uint4 hi, lo;
+          load8(gp + swz(t, (c & 31) >> 2), gp + swz(t, ((c & 31) >> 2) + 1), al);
+          load8(sm + LS::CEN + c * 4, sm + LS::CEN + c * 4 + 16, x);
+          unpack8(*reinterpret_cast<const uint4*>(sm + LS::KT + pn * 16384 + off), kk);
+#pragma unroll
+          for (int j = 0; j < 8; j++) al[j] = ex2(al[j] - x[j]);  // |exponent| < 100: no flush
           if (!krow) {
-            float qq[8], x[8], y[8], o[8];
-            uint4* qat = reinterpret_cast<uint4*>(sm + LS::QK + wg * 16384 + off);
-            unpack8(*qat, qq);
+            unpack8(*reinterpret_cast<const uint4*>(sm + LS::QK + pn * 16384 + off), x);
 #pragma unroll
             for (int j = 0; j < 8; j++) {
-              const float al = ex2(gg[j] - cen[j]);  // |exponent| < 100: no flush
-              x[j] = qq[j] * al;
-              y[j] = kk[j] * rcp(al);
+              kk[j] *= rcp(al[j]);
+              x[j] *= al[j];
             }
-            if (wide) {
-#pragma unroll
-              for (int j = 0; j < 8; j++) o[j] = qq[j] * exp2f(gg[j]);
-            } else {
-#pragma unroll
-              for (int j = 0; j < 8; j++) o[j] = (x[j] * e2[j]) * e2[j];
-            }
-            split8(x, hi, lo);
-            tmem_st4(tlane + TM_A + c / 2, hi);
-            tmem_st4(tlane + TM_A + 64 + c / 2, lo);
-            if (!wide) {  // the pairwise path below still reads q
-              *qat = pack8(o);
-            } else {
-              epk[c8] = pack8(o);
-            }
-            split8(y, hi, lo);
-            *reinterpret_cast<uint4*>(sm + LS::Y + wg * 8192 + off) = hi;
-            *reinterpret_cast<uint4*>(sm + LS::Y + 16384 + wg * 8192 + off) = lo;
+            split8(kk, hi, lo);
+            *reinterpret_cast<uint4*>(sm + LS::Y + pn * 8192 + off) = hi;
+            *reinterpret_cast<uint4*>(sm + LS::Y + 16384 + pn * 8192 + off) = lo;
           } else {
-            float gl[8], x[8], o[8], kg[8];
-            load8(sm + LS::GL + c * 4, sm + LS::GL + c * 4 + 16, gl);
-            float bb[8];
-            if (VB) unpack8(*reinterpret_cast<const uint4*>(p.bg + base128 + (size_t)t * ldt + c), bb);
+            if (VB) unpack8(*reinterpret_cast<const uint4*>(p.bg + base128 + (size_t)t * ldt + c), x);
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-              const float bk = (VB ? bb[j] : bs) * kk[j];
-              x[j] = bk * ex2(gg[j] - cen[j]);
-              kg[j] = kk[j] * ex2(gl[j] - gg[j]);
-              o[j] = bk;
-            }
-            if (wide) {
-#pragma unroll
-              for (int j = 0; j < 8; j++) o[j] *= exp2f(gg[j]);
-            } else {
-#pragma unroll
-              for (int j = 0; j < 8; j++) o[j] = (x[j] * e2[j]) * e2[j];
-            }
-            split8(x, hi, lo);
-            tmem_st4(tlane + TM_A + c / 2, hi);
-            tmem_st4(tlane + TM_A + 64 + c / 2, lo);
-            epk[c8] = pack8(o);
-            kpk[c8] = pack8(kg);
+            for (int j = 0; j < 8; j++) x[j] = (VB ? x[j] : bs) * kk[j] * al[j];
           }
+          split8(x, hi, lo);
+          tmem_st4(tlane + TM_A + c / 2, hi);
+          tmem_st4(tlane + TM_A + 64 + c / 2, lo);
         }
         tmem_st_wait();
       }
@@ -412,9 +400,7 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       __syncthreads();
       tc_fence_after_sync();
       if (wide) {
-        // exact pairwise sums over the tiles, thread = (row i, every fourth column j); the matrix to invert goes to
-        // the Yc region first (its place holds gate rows) and then to its place
-        float* tmp = reinterpret_cast<float*>(sm + LS::Y);
+        // exact pairwise sums over the tiles, thread = (row i, every fourth column j)
         const int i = tid >> 2;
         auto bfat = [&](uint32_t tile, int r, int k) {
           return bf2f(*reinterpret_cast<const bf16*>(sm + tile + (k >> 6) * 16384 + swz(r, (k & 63) >> 3) + (k & 7) * 2));
@@ -427,7 +413,6 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         for (int j = tid & 3; j < C; j += 4) {
           float aq = 0.f, ak = 0.f;
           if (j <= i) {
-#pragma unroll 4
             for (int k = 0; k < 128; k++) {
               const float f = exp2f(gat(i, k) - gat(j, k)) * bfat(LS::KT, j, k);
               aq = fmaf(bfat(LS::QK, i, k), f, aq);
@@ -435,15 +420,9 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             }
           }
           p.Aqk[base64 + (size_t)i * H * 64 + j] = f2bf(p.scale * aq);
-          tmp[i * C + j] = j < i ? ak : 0.f;
+          sL[i * LDL + j] = j < i ? ak : 0.f;
         }
-        __syncthreads();
-        for (int e = tid; e < C * C; e += TPB) sL[(e >> 6) * LDL + (e & 63)] = tmp[e];
-        if (!krow) {
-#pragma unroll
-          for (int c8 = 0; c8 < 8; c8++)
-            *reinterpret_cast<uint4*>(sm + LS::QK + wg * 16384 + swz(t, c8)) = epk[c8];
-        }
+        __syncthreads();  // the tiles are rewritten below
       } else if (warp == 0 && alive) {
         if (leader) {
 #pragma unroll
@@ -457,17 +436,9 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       if (leader) mma_commit(&bars[LB_D]);
       __syncwarp();
-      if (krow) {  // k and the gate rows are dead: E and kg take their places
-#pragma unroll
-        for (int c8 = 0; c8 < 8; c8++) {
-          *reinterpret_cast<uint4*>(sm + LS::KT + wg * 16384 + swz(t, c8)) = epk[c8];
-          *reinterpret_cast<uint4*>(sm + LS::KG + wg * 8192 + swz(t, c8)) = kpk[c8];
-        }
-      }
     } else {
       // ---- scalar gate / none: exact products on the tiles as they landed --------------------------------------
-      wait(LB_QG, 41);
-      wait(LB_K, 42);
+      wait(LB_QK, 42);
       if (warp == 0 && alive) {
         tc_fence_after_sync();
         if (leader) {
@@ -476,124 +447,121 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             mma_f16_lo(tb + TM_D, dl(LS::QK + (ks >> 2) * 16384 + (ks & 3) * 32, 16),
                        dl(LS::KT + (ks >> 2) * 16384 + (ks & 3) * 32, 16), ID_D, ks > 0);
           mma_commit(&bars[LB_D]);
-          if (GATE == GATE_NONE && p.write_qk) {  // qg = q, kg = k
-            for (int pn = 0; pn < 2; pn++) {
-              tma_store_2d(&tmQg, sm + LS::QK + pn * 16384, h * 128 + 64 * pn, row0);
-              tma_store_2d(&tmKg, sm + LS::KT + pn * 16384, h * 128 + 64 * pn, row0);
-            }
-            tma_store_commit();
-            tma_store_wait_read();  // before the barrier after which E takes the place of k
-          }
         }
         __syncwarp();
       }
+      __syncthreads();  // beta and gate rows visible
+      wait(LB_D, 43);   // k is rewritten in place below
     }
-    if (!VEC) __syncthreads();  // beta and gate rows visible; the copies of q and k have left
-    wait(LB_D, 43);
-    tc_fence_after_sync();
 
-    // ---- Aqk (rows of q) and L (rows of k): 32 columns per thread --------------------------------------------------
-    if (alive && !wide) {
-      uint32_t u[32];
-      tmem_ld32(tlane + TM_D + 32 * wg, u);
-      tmem_ld_wait();
-      float f0 = krow ? (VEC || VB ? 1.f : sBeta[t]) : p.scale;
-      uint32_t pk[4];
+    // ---- qg and kg in 16-byte pieces to global memory, E in place of k -----------------------------------------------
+    if (alive) {
+#pragma unroll 2
+      for (int i = tid; i < C * 16; i += TPB) {
+        const int r = i >> 4, c = (i & 15) * 8;
+        const uint32_t off = (c >> 6) * 16384 + swz(r, (c & 63) >> 3);
+        const size_t go = base128 + (size_t)r * ldt + c;
+        float kk[8], x[8], gam[8], kap[8];
+        uint4* kat = reinterpret_cast<uint4*>(sm + LS::KT + off);
+        const uint4 kraw = *kat, qraw = *reinterpret_cast<const uint4*>(sm + LS::QK + off);
+        unpack8(kraw, kk);
+        unpack8(qraw, x);
+        if (VEC) {
+          const unsigned char* gp = sm + LS::G + (c >> 5) * 8192;
+          load8(gp + swz(r, (c & 31) >> 2), gp + swz(r, ((c & 31) >> 2) + 1), gam);
+          load8(sm + LS::GL + c * 4, sm + LS::GL + c * 4 + 16, kap);
 #pragma unroll
-      for (int c = 0; c < 32; c += 4) {
-        float y[4];
+          for (int j = 0; j < 8; j++) {
+            kap[j] = ex2(kap[j] - gam[j]);
+            gam[j] = ex2(gam[j]);
+          }
+        } else if (GATE == GATE_SCALAR) {
+          const float g = ex2(sGs[r]), l = ex2(sGs[C - 1] - sGs[r]);
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const int col = 32 * wg + c + e;
-          const bool keep = krow ? col < t : col <= t;
-          float f = f0;
-          if (GATE == GATE_SCALAR) f *= exp2f(sGs[t] - sGs[keep ? col : t]);
-          y[e] = keep ? __uint_as_float(u[c + e]) * f : 0.f;
+          for (int j = 0; j < 8; j++) { gam[j] = g; kap[j] = l; }
         }
-        if (krow) {
-          *reinterpret_cast<float4*>(sL + t * LDL + 32 * wg + c) = make_float4(y[0], y[1], y[2], y[3]);
-        } else {
-          pk[(c >> 1) & 3] = pack_bf16(y[0], y[1]);
-          pk[((c >> 1) & 3) + 1] = pack_bf16(y[2], y[3]);
-          if (c & 4)
-            *reinterpret_cast<uint4*>(p.Aqk + base64 + (size_t)t * H * 64 + 32 * wg + c - 4) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        if (GATE != GATE_NONE) {
+          float y[8];
+#pragma unroll
+          for (int j = 0; j < 8; j++) { x[j] *= gam[j]; y[j] = kk[j] * kap[j]; }
+          *reinterpret_cast<uint4*>(p.qg + go) = pack8(x);
+          *reinterpret_cast<uint4*>(p.kg + go) = pack8(y);
+        } else if (p.write_qk) {
+          *reinterpret_cast<uint4*>(p.qg + go) = qraw;
+          *reinterpret_cast<uint4*>(p.kg + go) = kraw;
         }
+        if (VB) unpack8(*reinterpret_cast<const uint4*>(p.bg + go), x);
+        const float bs = VB ? 0.f : sBeta[r];
+#pragma unroll
+        for (int j = 0; j < 8; j++) kk[j] *= (VB ? x[j] : bs) * (GATE == GATE_NONE ? 1.f : gam[j]);
+        *kat = pack8(kk);
       }
     }
-    // ---- scalar gate / none: qg in place, E in place of k, kg ---------------------------------------------------------
-    if (!VEC && alive) {
+    if (VEC) wait(LB_D, 43);
+    tc_fence_after_sync();
+
+    // ---- Aqk (rows of q) and L (rows of k, over Yc) -------------------------------------------------------------------
+    if (alive && !wide) {
+      const float f0 = krow ? (VEC ? 1.f : sBeta[t]) : p.scale;
+#pragma unroll 1
+      for (int c0 = 64 / NG * wg; c0 < 64 / NG * (wg + 1); c0 += 16) {
+        float u[16];
+        tmem_ld16(tlane + TM_D + c0, u);
+        tmem_ld_wait();
 #pragma unroll
-      for (int it = 0; it < (C * 16) / TPB; it++) {
-        const int i = tid + it * TPB, r = i >> 4, c16 = i & 15;
-        const uint32_t off = (c16 >> 3) * 16384 + swz(r, c16 & 7);
-        const float bs = sBeta[r];
-        float kk[8], o[8];
-        unpack8(*reinterpret_cast<const uint4*>(sm + LS::KT + off), kk);
-        if (GATE == GATE_SCALAR) {
-          const float gam = exp2f(sGs[r]), kap = exp2f(sGs[C - 1] - sGs[r]);
-          float qq[8];
-          uint4* qat = reinterpret_cast<uint4*>(sm + LS::QK + off);
-          unpack8(*qat, qq);
-#pragma unroll
-          for (int j = 0; j < 8; j++) qq[j] *= gam;
-          *qat = pack8(qq);
-#pragma unroll
-          for (int j = 0; j < 8; j++) o[j] = kk[j] * kap;
-          *reinterpret_cast<uint4*>(sm + LS::KG + (c16 >> 3) * 8192 + swz(r, c16 & 7)) = pack8(o);
-#pragma unroll
-          for (int j = 0; j < 8; j++) o[j] = bs * kk[j] * gam;
-        } else {
-#pragma unroll
-          for (int j = 0; j < 8; j++) o[j] = bs * kk[j];
+        for (int e = 0; e < 16; e++) {
+          const int col = c0 + e;
+          const bool keep = krow ? col < t : col <= t;
+          float f = f0;
+          if (GATE == GATE_SCALAR) f *= ex2(sGs[t] - sGs[keep ? col : t]);
+          u[e] = keep ? u[e] * f : 0.f;
         }
-        *reinterpret_cast<uint4*>(sm + LS::KT + off) = pack8(o);
+        if (krow) {
+#pragma unroll
+          for (int e = 0; e < 16; e += 4)
+            *reinterpret_cast<float4*>(sL + t * LDL + c0 + e) = make_float4(u[e], u[e + 1], u[e + 2], u[e + 3]);
+        } else {
+          uint4* dst = reinterpret_cast<uint4*>(p.Aqk + base64 + (size_t)t * H * 64 + c0);
+          dst[0] = make_uint4(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]), pack_bf16(u[4], u[5]), pack_bf16(u[6], u[7]));
+          dst[1] = make_uint4(pack_bf16(u[8], u[9]), pack_bf16(u[10], u[11]), pack_bf16(u[12], u[13]), pack_bf16(u[14], u[15]));
+        }
       }
     }
     fence_async_smem();
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    if (leader && alive) {
-      if (VEC) load_v(chunk);  // Yc has been read
-      if (GATE != GATE_NONE) {
-        for (int pn = 0; pn < 2; pn++) {
-          tma_store_2d(&tmQg, sm + LS::QK + pn * 16384, h * 128 + 64 * pn, row0);
-          tma_store_2d(&tmKg, sm + LS::KG + pn * 8192, h * 128 + 64 * pn, row0);
-        }
-        tma_store_commit();
+    if (VEC) {
+      if (leader && alive) {  // q and the gate tile are dead
+        load_v(chunk);
+        if (next < p.total_chunks) load_g(next);
       }
+      __syncwarp();
     }
-    __syncwarp();
 
     invert_unit_lower(sL, tid);
 
     // ---- Akk: BF16, to global memory and twice into the operand tile; Z = w v in place --------------------------------
     {
-      const int i = tid >> 2, c0 = (tid & 3) * 16;
-      float x[16];
 #pragma unroll
-      for (int j = 0; j < 16; j += 4) {
-        const float4 f = *reinterpret_cast<const float4*>(sL + i * LDL + c0 + j);
-        x[j] = f.x; x[j + 1] = f.y; x[j + 2] = f.z; x[j + 3] = f.w;
-      }
-      uint32_t pk[8];
+      for (int e = tid; e < C * 8; e += TPB) {
+        const int i = e >> 3, c0 = (e & 7) * 8;
+        float x[8];
+        load8(reinterpret_cast<const unsigned char*>(sL + i * LDL + c0), reinterpret_cast<const unsigned char*>(sL + i * LDL + c0 + 4), x);
 #pragma unroll
-      for (int j = 0; j < 8; j++)
-        pk[j] = pack_bf16(c0 + 2 * j <= i ? x[2 * j] : 0.f, c0 + 2 * j + 1 <= i ? x[2 * j + 1] : 0.f);
-#pragma unroll
-      for (int half = 0; half < 2; half++) {
-        const uint4 v = make_uint4(pk[4 * half], pk[4 * half + 1], pk[4 * half + 2], pk[4 * half + 3]);
-        *reinterpret_cast<uint4*>(sm + LS::AK + swz(i, c0 / 8 + half)) = v;
-        *reinterpret_cast<uint4*>(sm + LS::AK + 8192 + swz(i, c0 / 8 + half)) = v;
-        *reinterpret_cast<uint4*>(p.Akk + base64 + (size_t)i * H * 64 + c0 + 8 * half) = v;
+        for (int j = 0; j < 8; j++) x[j] = c0 + j <= i ? x[j] : 0.f;
+        const uint4 v = pack8(x);
+        *reinterpret_cast<uint4*>(sm + LS::AK + swz(i, c0 / 8)) = v;
+        *reinterpret_cast<uint4*>(sm + LS::AK + 8192 + swz(i, c0 / 8)) = v;
+        *reinterpret_cast<uint4*>(p.Akk + base64 + (size_t)i * H * 64 + c0) = v;
       }
     }
     wait(LB_V, 44);
     if (alive) {
-#pragma unroll
-      for (int it = 0; it < (C * 16) / TPB; it++) {
-        const int i = tid + it * TPB, r = i >> 4, c16 = i & 15;
-        uint4* vat = reinterpret_cast<uint4*>(sm + LS::V + (c16 >> 3) * 8192 + swz(r, c16 & 7));
+#pragma unroll 2
+      for (int i = tid; i < C * 16; i += TPB) {
+        const int r = i >> 4, c16 = i & 15;
+        uint4* vat = reinterpret_cast<uint4*>(sm + VT + (c16 >> 3) * VP + swz(r, c16 & 7));
         float vv[8], ww[8];
         unpack8(*vat, vv);
         if (VB) unpack8(*reinterpret_cast<const uint4*>(p.wg + base128 + (size_t)r * ldt + c16 * 8), ww);
@@ -614,30 +582,27 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           mma_f16_lo(tb + TM_W, dl(LS::AK + ks * 32, 16), dl(LS::KT + ks * 2048, 16384), ID_WU, ks > 0);
 #pragma unroll
         for (int ks = 0; ks < 4; ks++)
-          mma_f16_lo(tb + TM_U, dl(LS::AK + ks * 32, 16), dl(LS::V + ks * 2048, 8192), ID_WU, ks > 0);
+          mma_f16_lo(tb + TM_U, dl(LS::AK + ks * 32, 16), dl(VT + ks * 2048, VP), ID_WU, ks > 0);
         mma_commit(&bars[LB_WU]);
-        // q, kg and the inverse are dead once the stores have read them: the next chunk's q and gate
-        tma_store_wait_read();
-        if (next < p.total_chunks) load_qg(next);
       }
       __syncwarp();
     }
     wait(LB_WU, 45);
     tc_fence_after_sync();
-    // ---- w (lanes 0..63) and u (64..127): 64 channels of row t into the dead E / Z tiles ------------------------------
+    // ---- w (lanes 0..63) and u (64..127): 32 channels of row t into the dead E / Z tiles ------------------------------
     if (alive) {
-      const uint32_t dst = krow ? LS::V + wg * 8192 : LS::KT + wg * 16384;
-#pragma unroll
-      for (int c = 0; c < 2; c++) {
-        uint32_t u[32];
-        tmem_ld32(tlane + (krow ? TM_U : TM_W) + 64 * wg + 32 * c, u);
+      const int c0 = wg * (128 / NG);
+      unsigned char* dst = sm + (krow ? VT + (c0 >> 6) * VP : LS::KT + (c0 >> 6) * 16384);
+#pragma unroll 1
+      for (int c = 0; c < 128 / NG; c += 16) {
+        float u[16], y[8];
+        tmem_ld16(tlane + (krow ? TM_U : TM_W) + c0 + c, u);
         tmem_ld_wait();
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-          float y[8];
+        for (int e = 0; e < 2; e++) {
 #pragma unroll
-          for (int j = 0; j < 8; j++) y[j] = __uint_as_float(u[8 * e + j]);
-          *reinterpret_cast<uint4*>(sm + dst + swz(t, 4 * c + e)) = pack8(y);
+          for (int j = 0; j < 8; j++) y[j] = u[8 * e + j];
+          *reinterpret_cast<uint4*>(dst + swz(t, ((c0 & 63) + c) / 8 + e)) = pack8(y);
         }
       }
     }
@@ -648,18 +613,17 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (leader && alive) {
       for (int pn = 0; pn < 2; pn++) {
         tma_store_2d(&tmW, sm + LS::KT + pn * 16384, h * 128 + 64 * pn, row0);
-        tma_store_2d(&tmU, sm + LS::V + pn * 8192, h * 128 + 64 * pn, row0);
+        tma_store_2d(&tmU, sm + VT + pn * VP, h * 128 + 64 * pn, row0);
       }
       tma_store_commit();
       tma_store_wait_read();
       if (next < p.total_chunks) {
-        load_k(next);
+        load_qk(next);
         if (!VEC) load_v(next);
       }
     }
     __syncwarp();
     ph ^= 1u;
-    // Yc of the next chunk is written over u: the wait for its k load (requested after u has left) covers that
   }
   if (leader) {
     if (!alive) {  // gave up: no copy or product may still be under way when the CTA exits
@@ -678,7 +642,7 @@ cudaError_t run(const CUtensorMap* tm, const LocalParams& p, cudaStream_t st) {
   if (e != cudaSuccess) return e;
   const int cap = 2 * 148;  // two CTAs per SM
   const int grid = p.total_chunks < cap ? p.total_chunks : cap;
-  chunk_fwd_tc_kernel<GATE, VB><<<grid, TPB, LS::TOTAL, st>>>(tm[0], tm[1], tm[2], tm[3], tm[4], tm[5], tm[6], tm[7], p);
+  chunk_fwd_tc_kernel<GATE, VB><<<grid, TPB, LS::TOTAL, st>>>(tm[0], tm[1], tm[2], tm[3], tm[4], tm[5], p);
   count_launch();
   return cudaGetLastError();
 }
@@ -689,17 +653,16 @@ cudaError_t launch_chunk_fwd_tc(const RewyFwdArgs& a, int* err, cudaStream_t st)
   const int B = a.B, T = a.T, H = a.H, NT = T / C;
   const uint64_t rows = (uint64_t)B * T, cols = (uint64_t)H * 128, pitch = (uint64_t)H * 256;
   const bool vector = gate_mode_of(a.family) == GATE_VECTOR;
-  CUtensorMap tm[8];
+  CUtensorMap tm[6];
   bool ok = encode_tmap_2d(&tm[0], a.q, 2, cols, rows, pitch, 64, 64) && encode_tmap_2d(&tm[1], a.k, 2, cols, rows, pitch, 64, 64) &&
-            encode_tmap_2d(&tm[2], a.v, 2, cols, rows, pitch, 64, 64) && encode_tmap_2d(&tm[4], a.qg, 2, cols, rows, pitch, 64, 64) &&
-            encode_tmap_2d(&tm[5], a.kg, 2, cols, rows, pitch, 64, 64) && encode_tmap_2d(&tm[6], a.w, 2, cols, rows, pitch, 64, 64) &&
-            encode_tmap_2d(&tm[7], a.u, 2, cols, rows, pitch, 64, 64);
+            encode_tmap_2d(&tm[2], a.v, 2, cols, rows, pitch, 64, 64) && encode_tmap_2d(&tm[4], a.w, 2, cols, rows, pitch, 64, 64) &&
+            encode_tmap_2d(&tm[5], a.u, 2, cols, rows, pitch, 64, 64);
   tm[3] = tm[0];  // never dereferenced without a vector gate
   if (ok && vector) ok = encode_tmap_panels(&tm[3], a.g, 4, cols, rows, (uint64_t)H * 512, 64, 4);
   if (!ok) return cudaErrorInvalidValue;
   LocalParams p;
   p.g = a.g; p.beta = a.beta; p.bg = (const bf16*)a.b_gate; p.wg = (const bf16*)a.w_gate;
-  p.Akk = (bf16*)a.Akk; p.Aqk = (bf16*)a.Aqk; p.err = err; p.T = T; p.H = H; p.NT = NT; p.total_chunks = B * H * NT;
+  p.Akk = (bf16*)a.Akk; p.Aqk = (bf16*)a.Aqk; p.qg = (bf16*)a.qg; p.kg = (bf16*)a.kg; p.err = err; p.T = T; p.H = H; p.NT = NT; p.total_chunks = B * H * NT;
   p.write_qk = a.qg != a.q || a.kg != a.k; p.scale = a.scale;
   switch (a.family) {
     case REWY_DELTA: return run<GATE_NONE, false>(tm, p, st);
