@@ -219,6 +219,34 @@ int rewy_gate_cumsum_fwd(const void* x, int x_is_f32, const float* A_log, const 
 int rewy_gate_act_bwd(const void* x, int x_is_f32, const float* A_log, const float* dt_bias, const float* dg, float* dx,
                       float* dA_part, float* dbias_part, int32_t B, int32_t T, int32_t H, rewy_stream_t stream);
 
+/* Row movement around the operators (no counterpart in the reference, whose release envelope rejects these inputs):
+ * lengths that are not multiples of 64 and grouped value heads.  A row map pairs the caller's B*T token rows with
+ * B*T_padded padded rows; packed sequences (B = 1) give device int32 [num_seqs + 1] offsets of both (the padded ones
+ * multiples of 64, the last equal to T_padded, the last of cu equal to T), else cu = cu_padded = NULL.
+ *   rewy_rows_pad / _cut       up to 8 tensors of row_bytes bytes per token row; padding rows get the 8-byte pattern `fill`
+ *   rewy_qk_front_fwd / _bwd   q, k BF16 [rows,H,128] -> yq, yk BF16 [padded rows, H*G, 128]: L2 normalisation if rq, rk
+ *                              (FP32 [padded rows, H]) are given, each head repeated G times; backward sums a group's dy
+ *                              (BF16 or FP32) in FP32 and writes dq, dk BF16 [rows,H,128]. */
+#define REWY_MAX_ROWS_ITEMS 8
+typedef struct RewyRowMap {
+  int32_t B, T, T_padded, num_seqs;
+  const int32_t* cu;
+  const int32_t* cu_padded;
+} RewyRowMap;
+typedef struct RewyRowsItem {
+  const void* src;
+  void* dst;
+  int64_t row_bytes;
+  uint64_t fill;
+} RewyRowsItem;
+int rewy_rows_pad(const RewyRowMap* map, const RewyRowsItem* items, int32_t n, rewy_stream_t stream);
+int rewy_rows_cut(const RewyRowMap* map, const RewyRowsItem* items, int32_t n, rewy_stream_t stream);
+int rewy_qk_front_fwd(const RewyRowMap* map, const void* q, const void* k, void* yq, void* yk, float* rq, float* rk,
+                      int32_t H, int32_t G, float eps, rewy_stream_t stream);
+int rewy_qk_front_bwd(const RewyRowMap* map, const void* yq, const void* yk, const float* rq, const float* rk,
+                      const void* dyq, const void* dyk, int32_t dy_is_f32, void* dq, void* dk, int32_t H, int32_t G,
+                      rewy_stream_t stream);
+
 /* Optional per-stage device timing of the whole-family calls (no counterpart in the reference, which
  * times stages by re-capturing them: research/operators/a800_ablation/audit.py:38-47).  While enabled, each
  * whole-family call records CUDA events on its stream around its stage launches (up to 256 calls).

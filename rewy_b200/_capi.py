@@ -25,6 +25,7 @@ EXPORTS = (
     "rewy_stage_chunk_adjoint_static", "rewy_static_device_status",
     "rewy_l2norm_fwd", "rewy_l2norm_bwd", "rewy_beta_sigmoid_fwd", "rewy_beta_sigmoid_bwd", "rewy_gate_cumsum_fwd",
     "rewy_gate_act_bwd", "rewy_chunk_fwd", "rewy_scalar_gate_cumsum_fwd", "rewy_set_forward_variant",
+    "rewy_rows_pad", "rewy_rows_cut", "rewy_qk_front_fwd", "rewy_qk_front_bwd",
     "rewy_last_error", "rewy_version", "rewy_kernel_launch_count",
 )
 
@@ -53,6 +54,15 @@ class FwdArgs(ctypes.Structure):
 
 class StageBuffers(ctypes.Structure):
     _fields_ = [(n, c_void_p) for n in ("w", "u", "qg", "kg", "v_new", "h", "Aqk", "dh", "dR", "dR_lo", "ctrl")]
+
+
+class RowMap(ctypes.Structure):
+    _fields_ = [("B", c_int32), ("T", c_int32), ("T_padded", c_int32), ("num_seqs", c_int32), ("cu", c_void_p),
+                ("cu_padded", c_void_p)]
+
+
+class RowsItem(ctypes.Structure):
+    _fields_ = [("src", c_void_p), ("dst", c_void_p), ("row_bytes", ctypes.c_int64), ("fill", ctypes.c_uint64)]
 
 
 _lib = None
@@ -104,6 +114,13 @@ def load():
                                       c_int32, c_int32, c_void_p]
     for name in ("rewy_l2norm_fwd", "rewy_l2norm_bwd", "rewy_beta_sigmoid_fwd", "rewy_beta_sigmoid_bwd",
                  "rewy_gate_cumsum_fwd", "rewy_gate_act_bwd"):
+        getattr(lib, name).restype = c_int
+    for name in ("rewy_rows_pad", "rewy_rows_cut"):
+        getattr(lib, name).argtypes = [ctypes.POINTER(RowMap), ctypes.POINTER(RowsItem), c_int32, c_void_p]
+    lib.rewy_qk_front_fwd.argtypes = [ctypes.POINTER(RowMap)] + [c_void_p] * 6 + [c_int32, c_int32, c_float, c_void_p]
+    lib.rewy_qk_front_bwd.argtypes = [ctypes.POINTER(RowMap)] + [c_void_p] * 6 + [c_int32, c_void_p, c_void_p, c_int32, c_int32,
+                                                                                  c_void_p]
+    for name in ("rewy_rows_pad", "rewy_rows_cut", "rewy_qk_front_fwd", "rewy_qk_front_bwd"):
         getattr(lib, name).restype = c_int
     lib.rewy_selftest_bounded_wait.argtypes = [c_void_p, c_void_p, ctypes.c_uint32, c_int, c_void_p]
     lib.rewy_selftest_bounded_wait.restype = c_int

@@ -28,6 +28,12 @@ def _as_input(x):
     return x.contiguous(), int(x.dtype == torch.float32)
 
 
+def _aligned(x):
+    """Contiguous and 16-byte aligned."""
+    x = x.contiguous()
+    return x if x.data_ptr() % 16 == 0 else x.clone()
+
+
 def l2norm_fwd(x, eps=1e-6):
     """x BF16 [..., 128] -> (y BF16, rstd FP32 [...])."""
     _need_cuda(x)
@@ -120,3 +126,75 @@ def gate_act_bwd(g_raw, A_log, dt_bias, dg):
                                                    _stream(g_raw)), "rewy_gate_act_bwd")
     # the per-(batch, chunk) partial sums are added up in a fixed order (deterministic), as FLA's kda_gate_bwd does
     return dx, dA_part.sum(0), (db_part.sum(0) if dt_bias is not None else None)
+
+
+def row_map(B, T, T_padded, cu=None, cu_padded=None):
+    """Pairs B*T token rows with B*T_padded padded rows; ``cu``, ``cu_padded``: device int32 offsets of packed sequences."""
+    m = _capi.RowMap()
+    m.B, m.T, m.T_padded = B, T, T_padded
+    if cu is not None:
+        m.cu, m.cu_padded, m.num_seqs = _capi.ptr(cu), _capi.ptr(cu_padded), cu.numel() - 1
+        m.keep = (cu, cu_padded)
+    return m
+
+
+def _pattern(fill, dtype):
+    """8 bytes of the fill value in `dtype`."""
+    if fill == 0:
+        return 0
+    one = torch.empty((), dtype=dtype).element_size()
+    return int.from_bytes(bytes(torch.full((8 // one,), fill, dtype=dtype).view(torch.uint8).tolist()), "little")
+
+
+def _move_rows(fn, tensors, fills, m, T_out):
+    _need_cuda(*tensors)
+    src = [t.contiguous() for t in tensors]
+    out = [torch.empty((t.shape[0], T_out) + tuple(t.shape[2:]), dtype=t.dtype, device=t.device) for t in src]
+    items = (_capi.RowsItem * len(src))()
+    for it, s, d, f in zip(items, src, out, fills):
+        it.src, it.dst, it.fill = _capi.ptr(s), _capi.ptr(d), _pattern(f, s.dtype)
+        it.row_bytes = s.numel() // (s.shape[0] * s.shape[1]) * s.element_size()
+    with torch.cuda.device(src[0].device):
+        _capi.check(getattr(_capi.load(), fn)(m, items, len(src), _stream(src[0])), fn)
+    return out
+
+
+def rows_pad(tensors, fills, m, T_padded):
+    """[B, T, ...] tensors of any element type -> [B, T_padded, ...], `fills` in the added rows; one launch."""
+    return _move_rows("rewy_rows_pad", tensors, fills, m, T_padded)
+
+
+def rows_cut(tensors, m, T):
+    """[B, T_padded, ...] -> [B, T, ...]; one launch."""
+    return _move_rows("rewy_rows_cut", tensors, [0] * len(tensors), m, T)
+
+
+def qk_front_fwd(q, k, m, groups, normalize, eps=1e-6):
+    """q, k BF16 [B,T,H,128] -> (BF16 [B,T_padded,H*groups,128] twice, rstd FP32 [B,T_padded,H] twice or None): L2
+    normalisation, padding rows and the repeat of every head in one pass."""
+    _need_cuda(q, k)
+    if q.dtype != torch.bfloat16 or k.dtype != torch.bfloat16 or q.shape[-1] != 128:
+        raise RuntimeError("rewy_b200 l2norm: expects BF16 rows of 128 values")
+    q, k = _aligned(q), _aligned(k)
+    B, _, H, _ = q.shape
+    y = [torch.empty(B, m.T_padded, H * groups, 128, dtype=q.dtype, device=q.device) for _ in (q, k)]
+    rstd = [torch.empty(B, m.T_padded, H, dtype=torch.float32, device=q.device) if normalize else None for _ in (q, k)]
+    with torch.cuda.device(q.device):
+        _capi.check(_capi.load().rewy_qk_front_fwd(m, _capi.ptr(q), _capi.ptr(k), _capi.ptr(y[0]), _capi.ptr(y[1]),
+                                                   _capi.ptr(rstd[0]), _capi.ptr(rstd[1]), H, groups, eps, _stream(q)),
+                    "rewy_qk_front_fwd")
+    return (*y, *rstd)
+
+
+def qk_front_bwd(yq, yk, rq, rk, dyq, dyk, m, groups):
+    """Backward of qk_front_fwd: dy BF16 or FP32 [B,T_padded,H*groups,128] -> dq, dk BF16 [B,T,H,128]."""
+    _need_cuda(yq, yk, dyq, dyk)
+    dyq, dyk = dyq.contiguous(), dyk.contiguous()
+    H = yq.shape[2] // groups
+    dq, dk = (torch.empty(yq.shape[0], m.T, H, 128, dtype=torch.bfloat16, device=yq.device) for _ in range(2))
+    with torch.cuda.device(yq.device):
+        _capi.check(_capi.load().rewy_qk_front_bwd(m, _capi.ptr(yq), _capi.ptr(yk), _capi.ptr(rq), _capi.ptr(rk),
+                                                   _capi.ptr(dyq), _capi.ptr(dyk), int(dyq.dtype == torch.float32),
+                                                   _capi.ptr(dq), _capi.ptr(dk), H, groups, _stream(yq)),
+                    "rewy_qk_front_bwd")
+    return dq, dk

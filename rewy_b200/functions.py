@@ -22,15 +22,34 @@ def _cumulative_gate(g, A_log=None, dt_bias=None):
     return _ew.gate_cumsum_fwd(g, A_log, dt_bias)
 
 
+def _front(q, k, rows, groups, normalize):
+    """q and k as the kernels take them: L2-normalised (optional), padded, each head repeated to its value heads, in one
+    pass.  Returns (q, k, q_rstd, k_rstd)."""
+    plain = groups == 1 and not rows.needed
+    if not normalize and (plain or q.dtype != torch.bfloat16):
+        return q, k, None, None   # (other types are refused by the forward)
+    if plain:   # every row where it is: the plain normalisation kernels are faster (B=2 T=4096 H=16: 31 + 47 against 35 + 58 us)
+        (q, q_rstd), (k, k_rstd) = _ew.l2norm_fwd(q), _ew.l2norm_fwd(k)
+        return q, k, q_rstd, k_rstd
+    return _ew.qk_front_fwd(q, k, rows.row_map(q.shape[0]), groups, normalize)
+
+
+def _front_backward(ctx, q, k, q_rstd, k_rstd, dq, dk):
+    if q_rstd is None and ctx.groups == 1:
+        return ctx.rows.cut_rows(dq, dk)
+    if ctx.groups == 1 and not ctx.rows.needed:
+        return _ew.l2norm_bwd(q, q_rstd, dq), _ew.l2norm_bwd(k, k_rstd, dk)
+    return _ew.qk_front_bwd(q, k, q_rstd, k_rstd, dq, dk, ctx.rows.row_map(q.shape[0]), ctx.groups)
+
+
 class ChunkKDAFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, g, beta, A_log, dt_bias, scale, initial_state, output_final_state, use_qk_l2norm_in_kernel,
                 use_gate_in_kernel, use_beta_sigmoid_in_kernel, allow_neg_eigval, disable_recompute, state_v_first,
-                cu_seqlens):
-        q_rstd = k_rstd = None
-        if use_qk_l2norm_in_kernel:
-            q, q_rstd = _ew.l2norm_fwd(q)
-            k, k_rstd = _ew.l2norm_fwd(k)
+                cu_seqlens, rows, groups):
+        q, k, q_rstd, k_rstd = _front(q, k, rows, groups, use_qk_l2norm_in_kernel)
+        # a raw gate input goes through -exp(A_log) softplus(g + dt_bias): a very negative value gives decay 0
+        v, beta, g = rows.pad_rows(v, beta, (g, -1e4 if use_gate_in_kernel else 0.0))
         beta_raw = beta
         if use_beta_sigmoid_in_kernel:
             beta = _ew.beta_sigmoid_fwd(beta_raw, 2.0 if allow_neg_eigval else 1.0)
@@ -47,38 +66,35 @@ class ChunkKDAFunction(torch.autograd.Function):
         ctx.scale, ctx.disable_recompute = scale, disable_recompute
         ctx.use_qk_l2norm_in_kernel, ctx.use_beta_sigmoid_in_kernel = use_qk_l2norm_in_kernel, use_beta_sigmoid_in_kernel
         ctx.use_gate_in_kernel, ctx.allow_neg_eigval, ctx.state_v_first = use_gate_in_kernel, allow_neg_eigval, state_v_first
-        return f["o"].type_as(q), f["final_state"]
+        ctx.rows, ctx.groups = rows, groups
+        return rows.cut_output(f["o"].type_as(q)), f["final_state"]
 
     @staticmethod
     def backward(ctx, do, dht):
         (q, q_rstd, k, k_rstd, v, g_cumsum, g_input, beta_raw, beta, A_log, dt_bias, Aqk, Akk, w, u, qg, kg, v_new, h,
          initial_state, cu_seqlens) = ctx.saved_tensors
         dq, dk, dv, db, dg, dh0, _, _ = _bwd.kda_backward(
-            q=q, k=k, v=v, beta=beta, Aqk=Aqk, Akk=Akk, scale=ctx.scale, initial_state=initial_state, do=do, dht=dht,
-            g=g_cumsum, state_v_first=ctx.state_v_first, cu_seqlens=cu_seqlens, disable_recompute=ctx.disable_recompute, w=w, u=u, qg=qg, kg=kg,
+            q=q, k=k, v=v, beta=beta, Aqk=Aqk, Akk=Akk, scale=ctx.scale, initial_state=initial_state,
+            do=ctx.rows.pad_output_grad(do), dht=dht, g=g_cumsum, state_v_first=ctx.state_v_first, cu_seqlens=cu_seqlens, disable_recompute=ctx.disable_recompute, w=w, u=u, qg=qg, kg=kg,
             v_new=v_new, h=h, out_dtype=torch.float32 if ctx.use_qk_l2norm_in_kernel else torch.bfloat16)
         dA = dbias = None
         if ctx.use_gate_in_kernel:
             dg, dA, dbias = _ew.gate_act_bwd(g_input, A_log, dt_bias, dg)
             dA = dA.view_as(A_log).to(A_log.dtype)
             dbias = None if dbias is None else dbias.view_as(dt_bias).to(dt_bias.dtype)
-        if ctx.use_qk_l2norm_in_kernel:
-            dq = _ew.l2norm_bwd(q, q_rstd, dq)
-            dk = _ew.l2norm_bwd(k, k_rstd, dk)
+        dq, dk = _front_backward(ctx, q, k, q_rstd, k_rstd, dq, dk)
         if ctx.use_beta_sigmoid_in_kernel:
             db = _ew.beta_sigmoid_bwd(beta_raw, db, 2.0 if ctx.allow_neg_eigval else 1.0)
-        return (dq.to(q), dk.to(k), dv.to(v), dg.to(g_input), db.to(beta_raw), dA, dbias, None, dh0, None, None, None,
-                None, None, None, None, None)
+        dv, dg, db = ctx.rows.cut_rows(dv, dg, db)
+        return (dq.to(q), dk.to(k), dv.to(v), dg.to(g_input), db.to(beta_raw), dA, dbias, None, dh0) + (None,) * 10
 
 
 class ChunkGDN2Function(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, g, b, w, scale, initial_state, output_final_state, use_qk_l2norm_in_kernel,
-                disable_recompute, state_v_first, cu_seqlens):
-        q_rstd = k_rstd = None
-        if use_qk_l2norm_in_kernel:
-            q, q_rstd = _ew.l2norm_fwd(q)
-            k, k_rstd = _ew.l2norm_fwd(k)
+                disable_recompute, state_v_first, cu_seqlens, rows, groups):
+        q, k, q_rstd, k_rstd = _front(q, k, rows, groups, use_qk_l2norm_in_kernel)
+        v, g, b, w = rows.pad_rows(v, g, b, w)
         g_cumsum = _cumulative_gate(g)
         f = chunk_forward("gdn2", q, k, v, g=g_cumsum, b=b, w=w, scale=scale, initial_state=initial_state,
                           output_final_state=output_final_state, g_is_cumsum=True, state_v_first=state_v_first,
@@ -89,32 +105,31 @@ class ChunkGDN2Function(torch.autograd.Function):
                               cu_seqlens)
         ctx.scale, ctx.disable_recompute, ctx.use_qk_l2norm_in_kernel = scale, disable_recompute, use_qk_l2norm_in_kernel
         ctx.state_v_first = state_v_first
-        return f["o"].type_as(q), f["final_state"]
+        ctx.rows, ctx.groups = rows, groups
+        return rows.cut_output(f["o"].type_as(q)), f["final_state"]
 
     @staticmethod
     def backward(ctx, do, dht):
         (q, q_rstd, k, k_rstd, v, g_cumsum, g_input, b, w, Aqk, Akk, w_wy, u_wy, qg, kg, v_new, h,
          initial_state, cu_seqlens) = ctx.saved_tensors
         dq, dk, dv, db, dw, dg, dh0, _, _ = _bwd.gdn2_backward(
-            q=q, k=k, v=v, b=b, w_gate=w, Aqk=Aqk, Akk=Akk, scale=ctx.scale, initial_state=initial_state, do=do,
+            q=q, k=k, v=v, b=b, w_gate=w, Aqk=Aqk, Akk=Akk, scale=ctx.scale, initial_state=initial_state,
+            do=ctx.rows.pad_output_grad(do),
             dht=dht, g=g_cumsum, state_v_first=ctx.state_v_first, cu_seqlens=cu_seqlens, w_wy=w_wy, u_wy=u_wy, qg=qg, kg=kg, v_new=v_new, h=h,
             disable_recompute=ctx.disable_recompute,
             out_dtype=torch.float32 if ctx.use_qk_l2norm_in_kernel else torch.bfloat16)
-        if ctx.use_qk_l2norm_in_kernel:
-            dq = _ew.l2norm_bwd(q, q_rstd, dq)
-            dk = _ew.l2norm_bwd(k, k_rstd, dk)
+        dq, dk = _front_backward(ctx, q, k, q_rstd, k_rstd, dq, dk)
+        dv, dg, db, dw = ctx.rows.cut_rows(dv, dg, db, dw)
         return (dq.to(q.dtype), dk.to(k.dtype), dv.to(v.dtype), dg.to(g_input.dtype), db.to(b.dtype), dw.to(w.dtype),
-                None, dh0, None, None, None, None, None)
+                None, dh0) + (None,) * 7
 
 
 class ChunkGatedDeltaRuleFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, g, beta, scale, initial_state, output_final_state, use_qk_l2norm_in_kernel,
-                use_beta_sigmoid_in_kernel, allow_neg_eigval, state_v_first, cu_seqlens):
-        q_rstd = k_rstd = None
-        if use_qk_l2norm_in_kernel:
-            q, q_rstd = _ew.l2norm_fwd(q)
-            k, k_rstd = _ew.l2norm_fwd(k)
+                use_beta_sigmoid_in_kernel, allow_neg_eigval, state_v_first, cu_seqlens, rows, groups):
+        q, k, q_rstd, k_rstd = _front(q, k, rows, groups, use_qk_l2norm_in_kernel)
+        v, g, beta = rows.pad_rows(v, g, beta)
         beta_raw = beta
         if use_beta_sigmoid_in_kernel:
             beta = _ew.beta_sigmoid_fwd(beta_raw, 2.0 if allow_neg_eigval else 1.0)
@@ -124,48 +139,48 @@ class ChunkGatedDeltaRuleFunction(torch.autograd.Function):
         ctx.scale, ctx.use_qk_l2norm_in_kernel = scale, use_qk_l2norm_in_kernel
         ctx.use_beta_sigmoid_in_kernel, ctx.allow_neg_eigval = use_beta_sigmoid_in_kernel, allow_neg_eigval
         ctx.state_v_first = state_v_first
-        return f["o"].to(q.dtype), f["final_state"]
+        ctx.rows, ctx.groups = rows, groups
+        return rows.cut_output(f["o"].to(q.dtype)), f["final_state"]
 
     @staticmethod
     def backward(ctx, do, dht):
         q, q_rstd, k, k_rstd, v, g, g_input, beta_raw, beta, A, initial_state, cu_seqlens = ctx.saved_tensors
         dq, dk, dv, db, dg, dh0, _, _ = _bwd.gdn_backward(
-            q=q, k=k, v=v, g=g, beta=beta, A=A, scale=ctx.scale, initial_state=initial_state, do=do, dht=dht,
+            q=q, k=k, v=v, g=g, beta=beta, A=A, scale=ctx.scale, initial_state=initial_state,
+            do=ctx.rows.pad_output_grad(do), dht=dht,
             state_v_first=ctx.state_v_first, cu_seqlens=cu_seqlens,
             out_dtype=torch.float32 if ctx.use_qk_l2norm_in_kernel else torch.bfloat16)
-        if ctx.use_qk_l2norm_in_kernel:
-            dq = _ew.l2norm_bwd(q, q_rstd, dq)
-            dk = _ew.l2norm_bwd(k, k_rstd, dk)
+        dq, dk = _front_backward(ctx, q, k, q_rstd, k_rstd, dq, dk)
         if ctx.use_beta_sigmoid_in_kernel:
             db = _ew.beta_sigmoid_bwd(beta_raw, db, 2.0 if ctx.allow_neg_eigval else 1.0)
-        return (dq.to(q), dk.to(k), dv.to(v), dg.to(g_input), db.to(beta_raw), None, dh0, None, None, None, None, None,
-                None)
+        dv, dg, db = ctx.rows.cut_rows(dv, dg, db)
+        return (dq.to(q), dk.to(k), dv.to(v), dg.to(g_input), db.to(beta_raw), None, dh0) + (None,) * 8
 
 
 class ChunkDeltaRuleFunction(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, q, k, v, beta, scale, initial_state, output_final_state, use_qk_l2norm_in_kernel, cu_seqlens):
-        q_rstd = k_rstd = None
-        if use_qk_l2norm_in_kernel:
-            q, q_rstd = _ew.l2norm_fwd(q)
-            k, k_rstd = _ew.l2norm_fwd(k)
+    def forward(ctx, q, k, v, beta, scale, initial_state, output_final_state, use_qk_l2norm_in_kernel, cu_seqlens, rows,
+                groups):
+        q, k, q_rstd, k_rstd = _front(q, k, rows, groups, use_qk_l2norm_in_kernel)
+        v, beta = rows.pad_rows(v, beta)
         f = chunk_forward("delta", q, k, v, beta=beta, scale=scale, initial_state=initial_state,
                           output_final_state=output_final_state, cu_seqlens=cu_seqlens)
         ctx.save_for_backward(q, q_rstd, k, k_rstd, v, beta, f["Akk"], initial_state, cu_seqlens)
         ctx.scale, ctx.use_qk_l2norm_in_kernel = scale, use_qk_l2norm_in_kernel
-        return f["o"].to(q.dtype), f["final_state"]
+        ctx.rows, ctx.groups = rows, groups
+        return rows.cut_output(f["o"].to(q.dtype)), f["final_state"]
 
     @staticmethod
     def backward(ctx, do, dht):
         q, q_rstd, k, k_rstd, v, beta, A, initial_state, cu_seqlens = ctx.saved_tensors
         dq, dk, dv, db, dh0 = _bwd.delta_backward(
-            q=q, k=k, v=v, beta=beta, A=A, scale=ctx.scale, initial_state=initial_state, do=do, dht=dht,
+            q=q, k=k, v=v, beta=beta, A=A, scale=ctx.scale, initial_state=initial_state,
+            do=ctx.rows.pad_output_grad(do), dht=dht,
             cu_seqlens=cu_seqlens,
             out_dtype=torch.float32 if ctx.use_qk_l2norm_in_kernel else torch.bfloat16)
-        if ctx.use_qk_l2norm_in_kernel:
-            dq = _ew.l2norm_bwd(q, q_rstd, dq)
-            dk = _ew.l2norm_bwd(k, k_rstd, dk)
-        return dq.to(q.dtype), dk.to(k.dtype), dv.to(v.dtype), db.to(beta.dtype), None, dh0, None, None, None
+        dq, dk = _front_backward(ctx, q, k, q_rstd, k_rstd, dq, dk)
+        dv, db = ctx.rows.cut_rows(dv, db)
+        return (dq.to(q.dtype), dk.to(k.dtype), dv.to(v.dtype), db.to(beta.dtype), None, dh0) + (None,) * 5
 
 
 def _packed(cu_seqlens, q):
@@ -177,12 +192,13 @@ def _packed(cu_seqlens, q):
 class _Ragged:
     """Lengths that are not multiples of the chunk: every sequence is extended to the next multiple of 64 by neutral
     tokens (q = k = v = 0, no decay), which change neither the state nor any real token's output, and the results are
-    cut back.  The padding and the cut are ordinary differentiable tensor operations around the autograd function, so
-    the gradients of the real tokens come out by themselves.  FLA handles such lengths by bounds checks inside its
-    kernels (the reference's release envelope rejects them: src/fast_delta_rule/runtime.py:87-88)."""
+    cut back.  The autograd functions do both with the library's row kernels (``pad_rows``, ``cut_rows``, and the q/k
+    front pass); ``pad`` and ``cut`` state the same as differentiable tensor operations for any device.  FLA handles
+    such lengths by bounds checks inside its kernels (the reference's release envelope rejects them:
+    src/fast_delta_rule/runtime.py:87-88)."""
 
     def __init__(self, T, device, cu_seqlens=None, cu_seqlens_cpu=None):
-        self.T, self.index, self.cu = T, None, None
+        self.T, self.cu, self._lengths = T, None, None
         if cu_seqlens is None:
             self.total = -(-T // 64) * 64
             self.needed = self.total != T
@@ -192,17 +208,57 @@ class _Ragged:
         padded = (lengths + 63) // 64 * 64
         self.needed = bool((padded != lengths).any())
         if not self.needed:
+            self.total = T
             return
-        starts = torch.cumsum(padded, 0) - padded
-        self.total = int(padded.sum())
-        self.index = torch.cat([torch.arange(int(n)) + int(s) for n, s in zip(lengths, starts)]).to(device)
-        self.cu = torch.cat([starts, starts[-1:] + padded[-1:]]).to(device=device, dtype=torch.int32)
+        self.total, self._lengths = int(padded.sum()), lengths
+        both = torch.zeros(2, host.numel(), dtype=torch.int32)
+        both[0, 1:] = torch.cumsum(lengths, 0)
+        both[1, 1:] = torch.cumsum(padded, 0)
+        self._cu_real, self.cu = both.to(device)
+
+    def row_map(self, B):
+        return _ew.row_map(B, self.T, self.total, None if self.cu is None else self._cu_real, self.cu)
+
+    def pad_rows(self, *tensors):
+        """[B, T, ...] tensors, or (tensor, fill value) pairs -> [B, padded T, ...]; one launch for all of them."""
+        pairs = [t if isinstance(t, tuple) else (t, 0.0) for t in tensors]
+        if not self.needed:
+            out = [t for t, _ in pairs]
+        else:
+            out = _ew.rows_pad([t for t, _ in pairs], [f for _, f in pairs], self.row_map(pairs[0][0].shape[0]), self.total)
+        return out[0] if len(out) == 1 else out
+
+    def cut_rows(self, *tensors):
+        """The inverse; for a fixed batch views of the padded tensors."""
+        if not self.needed:
+            out = tensors
+        elif self.cu is None:
+            out = tuple(t[:, :self.T] for t in tensors)
+        else:
+            out = _ew.rows_cut(tensors, self.row_map(1), self.T)
+        return out[0] if len(out) == 1 else out
+
+    # The output of a fixed batch is cut outside the autograd function, as a view that may be written in place like any
+    # other; a packed one is gathered inside.
+    def cut_output(self, o):
+        return o if self.cu is None else self.cut_rows(o)
+
+    def pad_output_grad(self, do):
+        return do if self.cu is None else self.pad_rows(do)
+
+    @property
+    def index(self):
+        """Padded row of every token of a packed batch."""
+        if self._lengths is None:
+            return None
+        starts = self.cu[:-1].cpu().to(torch.int64)
+        return torch.cat([torch.arange(int(n)) + int(s) for n, s in zip(self._lengths, starts)]).to(self.cu.device)
 
     def pad(self, x, fill=0.0):
         """x [B, T, ...] -> [B, padded T, ...]"""
         if x is None or not self.needed:
             return x
-        if self.index is None:
+        if self.cu is None:
             tail = x.new_full((x.shape[0], self.total - self.T) + tuple(x.shape[2:]), fill)
             return torch.cat([x, tail], 1)
         return x.new_full((x.shape[0], self.total) + tuple(x.shape[2:]), fill).index_copy(1, self.index, x)
@@ -210,7 +266,7 @@ class _Ragged:
     def cut(self, o):
         if not self.needed:
             return o
-        return o[:, :self.T] if self.index is None else o.index_select(1, self.index)
+        return o[:, :self.T] if self.cu is None else o.index_select(1, self.index)
 
 
 def _common_checks(q, k, v, initial_state):
@@ -253,12 +309,11 @@ class _Narrow:
         return o[..., :self.V], final_state
 
 
-def _grouped(q, k, v):
-    """Grouped value heads (HV = G * H; value head hv reads query/key head hv // G, as in FLA's kernels): q and k are
-    repeated to HV heads, and autograd's backward of the repeat sums dq and dk over each group.  The kernels then see
-    equal head counts; the price is G copies of q and k."""
-    G = v.shape[2] // q.shape[2]
-    return (q, k) if G == 1 else (q.repeat_interleave(G, 2), k.repeat_interleave(G, 2))
+def _groups(q, v):
+    """Grouped value heads (HV = G * H; value head hv reads query/key head hv // G, as in FLA's kernels): the front pass
+    repeats q and k to HV heads and its backward sums dq and dk over each group, so the kernels see equal head counts;
+    the price is G copies of q and k."""
+    return v.shape[2] // q.shape[2]
 
 
 @torch.compiler.disable
@@ -286,16 +341,14 @@ def chunk_kda(q, k, v, g, beta, scale=None, initial_state=None, output_final_sta
         if use_gate_in_kernel:
             raise ValueError("rewy_b200 chunk_kda: the fused gate needs K = 128 (dt_bias is laid out per channel)")
         q, k, g, v, initial_state = nw.key(q), nw.key(k), nw.key(g), nw.value(v), nw.state(initial_state, state_v_first)
-    q, k = _grouped(q, k, v)
     rg = _Ragged(q.shape[1], q.device, cu_seqlens, cu_seqlens_cpu)
     if rg.needed:
-        # a raw gate input goes through -exp(A_log) softplus(g + dt_bias): a very negative value gives decay 0
-        q, k, v, beta, g = rg.pad(q), rg.pad(k), rg.pad(v), rg.pad(beta), rg.pad(g, -1e4 if use_gate_in_kernel else 0.0)
         cu_seqlens = rg.cu
     o, final_state = ChunkKDAFunction.apply(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, output_final_state,
                                             use_qk_l2norm_in_kernel, use_gate_in_kernel, use_beta_sigmoid_in_kernel,
-                                            allow_neg_eigval, disable_recompute, state_v_first, _packed(cu_seqlens, q))
-    return nw.cut(rg.cut(o), final_state, state_v_first)
+                                            allow_neg_eigval, disable_recompute, state_v_first, _packed(cu_seqlens, q), rg,
+                                            _groups(q, v))
+    return nw.cut(o if rg.cu is not None else rg.cut(o), final_state, state_v_first)
 
 
 @torch.compiler.disable
@@ -311,15 +364,14 @@ def chunk_gdn2(q, k, v, g, b, w, scale=None, initial_state=None, output_final_st
     if nw.needed:
         q, k, g, b = nw.key(q), nw.key(k), nw.key(g), nw.key(b)
         v, w, initial_state = nw.value(v), nw.value(w), nw.state(initial_state, state_v_first)
-    q, k = _grouped(q, k, v)
     rg = _Ragged(q.shape[1], q.device, cu_seqlens, cu_seqlens_cpu)
     if rg.needed:
-        q, k, v, g, b, w = (rg.pad(x) for x in (q, k, v, g, b, w))
         cu_seqlens = rg.cu
     o, final_state = ChunkGDN2Function.apply(q, k, v, g, b, w, scale, initial_state, output_final_state,
                                              use_qk_l2norm_in_kernel, disable_recompute, state_v_first,
-                                             _packed(cu_seqlens, q))
-    return nw.cut(rg.cut(o), final_state, state_v_first)
+                                             _packed(cu_seqlens, q), rg,
+                                            _groups(q, v))
+    return nw.cut(o if rg.cu is not None else rg.cut(o), final_state, state_v_first)
 
 
 @torch.compiler.disable
@@ -334,15 +386,14 @@ def chunk_gated_delta_rule(q, k, v, g, beta, scale=None, initial_state=None, out
     nw = _Narrow(q, v)
     if nw.needed:
         q, k, v, initial_state = nw.key(q), nw.key(k), nw.value(v), nw.state(initial_state, state_v_first)
-    q, k = _grouped(q, k, v)
     rg = _Ragged(q.shape[1], q.device, cu_seqlens, cu_seqlens_cpu)
     if rg.needed:
-        q, k, v, g, beta = (rg.pad(x) for x in (q, k, v, g, beta))
         cu_seqlens = rg.cu
     o, final_state = ChunkGatedDeltaRuleFunction.apply(q, k, v, g, beta, scale, initial_state, output_final_state,
                                                        use_qk_l2norm_in_kernel, use_beta_sigmoid_in_kernel,
-                                                       allow_neg_eigval, state_v_first, _packed(cu_seqlens, q))
-    return nw.cut(rg.cut(o), final_state, state_v_first)
+                                                       allow_neg_eigval, state_v_first, _packed(cu_seqlens, q), rg,
+                                            _groups(q, v))
+    return nw.cut(o if rg.cu is not None else rg.cut(o), final_state, state_v_first)
 
 
 @torch.compiler.disable
@@ -355,11 +406,10 @@ def chunk_delta_rule(q, k, v, beta, scale=None, initial_state=None, output_final
     nw = _Narrow(q, v)
     if nw.needed:
         q, k, v, initial_state = nw.key(q), nw.key(k), nw.value(v), nw.state(initial_state)
-    q, k = _grouped(q, k, v)
     rg = _Ragged(q.shape[1], q.device, cu_seqlens, cu_seqlens_cpu)
     if rg.needed:
-        q, k, v, beta = (rg.pad(x) for x in (q, k, v, beta))
         cu_seqlens = rg.cu
     o, final_state = ChunkDeltaRuleFunction.apply(q, k, v, beta, scale, initial_state, output_final_state,
-                                                  use_qk_l2norm_in_kernel, _packed(cu_seqlens, q))
-    return nw.cut(rg.cut(o), final_state)
+                                                  use_qk_l2norm_in_kernel, _packed(cu_seqlens, q), rg,
+                                            _groups(q, v))
+    return nw.cut(o if rg.cu is not None else rg.cut(o), final_state)
