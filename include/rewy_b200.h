@@ -218,6 +218,9 @@ int rewy_gate_cumsum_fwd(const void* x, int x_is_f32, const float* A_log, const 
                          float* g_act, int32_t B, int32_t T, int32_t H, rewy_stream_t stream);
 int rewy_gate_act_bwd(const void* x, int x_is_f32, const float* A_log, const float* dt_bias, const float* dg, float* dx,
                       float* dA_part, float* dbias_part, int32_t B, int32_t T, int32_t H, rewy_stream_t stream);
+/* The same with dx rounded to BF16 (the input's type) in the same pass. */
+int rewy_gate_act_bwd_bf16(const void* x, int x_is_f32, const float* A_log, const float* dt_bias, const float* dg, void* dx,
+                           float* dA_part, float* dbias_part, int32_t B, int32_t T, int32_t H, rewy_stream_t stream);
 
 /* Row movement around the operators (no counterpart in the reference, whose release envelope rejects these inputs):
  * lengths that are not multiples of 64 and grouped value heads.  A row map pairs the caller's B*T token rows with

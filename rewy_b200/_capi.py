@@ -24,7 +24,7 @@ EXPORTS = (
     "rewy_set_prepare_variant", "rewy_set_scan_overlap",
     "rewy_stage_chunk_adjoint_static", "rewy_static_device_status",
     "rewy_l2norm_fwd", "rewy_l2norm_bwd", "rewy_beta_sigmoid_fwd", "rewy_beta_sigmoid_bwd", "rewy_gate_cumsum_fwd",
-    "rewy_gate_act_bwd", "rewy_chunk_fwd", "rewy_scalar_gate_cumsum_fwd", "rewy_set_forward_variant",
+    "rewy_gate_act_bwd", "rewy_gate_act_bwd_bf16", "rewy_chunk_fwd", "rewy_scalar_gate_cumsum_fwd", "rewy_set_forward_variant",
     "rewy_rows_pad", "rewy_rows_cut", "rewy_qk_front_fwd", "rewy_qk_front_bwd",
     "rewy_last_error", "rewy_version", "rewy_kernel_launch_count",
 )
@@ -110,10 +110,10 @@ def load():
     lib.rewy_beta_sigmoid_bwd.argtypes = [c_void_p, c_int, c_void_p, c_void_p, i64, c_float, c_void_p]
     lib.rewy_gate_cumsum_fwd.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32,
                                          c_void_p]
-    lib.rewy_gate_act_bwd.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32,
+    lib.rewy_gate_act_bwd_bf16.argtypes = lib.rewy_gate_act_bwd.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32,
                                       c_int32, c_int32, c_void_p]
     for name in ("rewy_l2norm_fwd", "rewy_l2norm_bwd", "rewy_beta_sigmoid_fwd", "rewy_beta_sigmoid_bwd",
-                 "rewy_gate_cumsum_fwd", "rewy_gate_act_bwd"):
+                 "rewy_gate_cumsum_fwd", "rewy_gate_act_bwd", "rewy_gate_act_bwd_bf16"):
         getattr(lib, name).restype = c_int
     for name in ("rewy_rows_pad", "rewy_rows_cut"):
         getattr(lib, name).argtypes = [ctypes.POINTER(RowMap), ctypes.POINTER(RowsItem), c_int32, c_void_p]

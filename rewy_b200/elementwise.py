@@ -107,9 +107,9 @@ def gate_cumsum_fwd(g, A_log=None, dt_bias=None):
     return out
 
 
-def gate_act_bwd(g_raw, A_log, dt_bias, dg):
+def gate_act_bwd(g_raw, A_log, dt_bias, dg, out_dtype=torch.float32):
     """Backward of the KDA gate activation.  dg: FP32 gradient of the activated per-step gate.
-    Returns (dg_raw FP32 [B,T,H,128], dA_log FP32 [H], ddt_bias FP32 [H*128] or None)."""
+    Returns (dg_raw [B,T,H,128] in ``out_dtype``: FP32 or BF16, dA_log FP32 [H], ddt_bias FP32 [H*128] or None)."""
     _need_cuda(g_raw, A_log, dt_bias, dg)
     B, T, H, K = g_raw.shape
     gin, is_f32 = _as_input(g_raw)
@@ -117,13 +117,14 @@ def gate_act_bwd(g_raw, A_log, dt_bias, dg):
     a = A_log.float().contiguous().view(-1)
     bias = None if dt_bias is None else dt_bias.float().contiguous().view(-1)
     nt = T // 64
-    dx = torch.empty(gin.shape, dtype=torch.float32, device=g_raw.device)
+    dx = torch.empty(gin.shape, dtype=out_dtype, device=g_raw.device)
+    fn = "rewy_gate_act_bwd_bf16" if out_dtype == torch.bfloat16 else "rewy_gate_act_bwd"
     dA_part = torch.empty(B * nt, H, dtype=torch.float32, device=g_raw.device)
     db_part = torch.empty(B * nt, H * 128, dtype=torch.float32, device=g_raw.device)
     with torch.cuda.device(g_raw.device):
-        _capi.check(_capi.load().rewy_gate_act_bwd(_capi.ptr(gin), is_f32, _capi.ptr(a), _capi.ptr(bias), _capi.ptr(dg),
-                                                   _capi.ptr(dx), _capi.ptr(dA_part), _capi.ptr(db_part), B, T, H,
-                                                   _stream(g_raw)), "rewy_gate_act_bwd")
+        _capi.check(getattr(_capi.load(), fn)(_capi.ptr(gin), is_f32, _capi.ptr(a), _capi.ptr(bias), _capi.ptr(dg),
+                                              _capi.ptr(dx), _capi.ptr(dA_part), _capi.ptr(db_part), B, T, H,
+                                              _stream(g_raw)), fn)
     # the per-(batch, chunk) partial sums are added up in a fixed order (deterministic), as FLA's kda_gate_bwd does
     return dx, dA_part.sum(0), (db_part.sum(0) if dt_bias is not None else None)
 

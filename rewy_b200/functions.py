@@ -79,7 +79,8 @@ class ChunkKDAFunction(torch.autograd.Function):
             v_new=v_new, h=h, out_dtype=torch.float32 if ctx.use_qk_l2norm_in_kernel else torch.bfloat16)
         dA = dbias = None
         if ctx.use_gate_in_kernel:
-            dg, dA, dbias = _ew.gate_act_bwd(g_input, A_log, dt_bias, dg)
+            dg, dA, dbias = _ew.gate_act_bwd(g_input, A_log, dt_bias, dg,
+                                              torch.bfloat16 if g_input.dtype == torch.bfloat16 else torch.float32)
             dA = dA.view_as(A_log).to(A_log.dtype)
             dbias = None if dbias is None else dbias.view_as(dt_bias).to(dt_bias.dtype)
         dq, dk = _front_backward(ctx, q, k, q_rstd, k_rstd, dq, dk)
