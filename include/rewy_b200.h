@@ -154,6 +154,7 @@ int rewy_stage_chunk_adjoint(const RewyBwdArgs* args, const RewyStageBuffers* bu
  * writes the output o, the final state and the whole saved set of the backward.  Three launches on the stream: the
  * chunk-local kernel (Akk, Aqk, w, u, qg, kg), the forward state scan (h, v_new, final state) and the output kernel.
  * g is the chunk-local cumulative gate in log2 units (rewy_gate_cumsum_fwd / rewy_scalar_gate_cumsum_fwd write it).
+ * Without a gate (DeltaNet) qg = q and kg = k: the caller may pass q and k themselves there, and nothing is written.
  * Every output pointer except final_state is required; ctrl is an int32[2] control block whose first word is the
  * device status word (rewy_device_status). */
 typedef struct RewyFwdArgs {

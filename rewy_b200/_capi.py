@@ -10,6 +10,7 @@ from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 LIB_PATH = PKG / "librewy_b200.so"
+TORCH_LIB_PATH = PKG / "rewy_b200_torch.so"   # torch operators over it (csrc/binding.cpp)
 
 DELTA, GDN, KDA, GDN2 = 0, 1, 2, 3
 FAMILY_ID = {"delta": DELTA, "gdn": GDN, "kda": KDA, "gdn2": GDN2}
@@ -144,6 +145,22 @@ def load():
     lib.rewy_version.restype = c_char_p
     lib.rewy_kernel_launch_count.restype = c_int
     _lib = lib
+    return lib
+
+
+_torch_lib_loaded = False
+
+
+def load_torch():
+    """Load the library and the torch operators over it once; returns the library."""
+    global _torch_lib_loaded
+    lib = load()
+    if not _torch_lib_loaded:
+        import torch
+        if not TORCH_LIB_PATH.exists():
+            raise RuntimeError(f"{TORCH_LIB_PATH} is missing: build it with `python -m rewy_b200.build`")
+        torch.ops.load_library(str(TORCH_LIB_PATH))
+        _torch_lib_loaded = True
     return lib
 
 

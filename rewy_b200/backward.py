@@ -8,76 +8,33 @@ delta.py:125-138).  All arithmetic happens in librewy_b200.so; this module only 
 allocates outputs and workspace with torch and marshals raw pointers.
 
 The call into the library is a torch custom operator, ``torch.ops.rewy_b200.family_bwd`` (registered with
-``torch.library`` for CUDA tensors, with a shape-only fake implementation): the four functions below are
+``torch.library`` for CUDA tensors, with a shape-only fake implementation; csrc/binding.cpp): the four functions below are
 thin bindings of it, so the backward is a single opaque node for ``torch.compile`` / export, and the C ABI
 stays the only thing underneath.
 """
-from typing import Optional
-
 import torch
-from torch import Tensor
 
 from . import _capi
 from .runtime import record
 
-_FAMILY_FN = {_capi.KDA: "rewy_kda_bwd", _capi.GDN2: "rewy_gdn2_bwd", _capi.GDN: "rewy_gdn_bwd",
-              _capi.DELTA: "rewy_delta_bwd"}
-_NONE = None
+# The operator is defined here and implemented in csrc/binding.cpp (CUDA; differentiating through it raises).  It gives
+# (dq, dk, dv, dg, dbeta, db_gate, dw_gate, dh0); outputs a family does not have are empty tensors.  Tensors must be
+# contiguous, on one CUDA device, in the dtypes of RewyBwdArgs.
+_ops = torch.library.Library("rewy_b200", "DEF")
+_ops.define(
+    "family_bwd(int family, int policy, bool out_f32, int intra_passes, bool state_v_first, float scale, Tensor q, Tensor k, "
+    "Tensor v, Tensor d_o, Tensor Akk, Tensor(a!) workspace, Tensor? g, Tensor? beta, Tensor? b_gate, Tensor? w_gate, "
+    "Tensor? Aqk, Tensor? h0, Tensor? dht, Tensor? w, Tensor? qg, Tensor? kg, Tensor? v_new, Tensor? h, Tensor? cu_seqlens) "
+    "-> (Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor)", tags=(torch.Tag.needs_fixed_stride_order,))
+_ops.define(   # no gradient formula and no fake implementation: chunk_forward is the only caller, under no_grad
+    "chunk_fwd(int family, bool state_v_first, bool output_final_state, float scale, Tensor q, Tensor k, Tensor v, Tensor? g, "
+    "Tensor? beta, Tensor? b_gate, Tensor? w_gate, Tensor? h0, Tensor? cu_seqlens) -> (Tensor, Tensor, Tensor, Tensor, Tensor, "
+    "Tensor, Tensor, Tensor, Tensor, Tensor, Tensor)")
+if _capi.TORCH_LIB_PATH.exists():
+    _capi.load_torch()
 
 
-def _empty(dev):
-    return torch.empty(0, device=dev)
-
-
-@torch.library.custom_op("rewy_b200::family_bwd", mutates_args=("workspace",), device_types="cuda")
-def _family_bwd(family: int, policy: int, out_f32: bool, intra_passes: int, state_v_first: bool, scale: float,
-                q: Tensor, k: Tensor, v: Tensor, d_o: Tensor, Akk: Tensor, workspace: Tensor,
-                g: Optional[Tensor], beta: Optional[Tensor], b_gate: Optional[Tensor], w_gate: Optional[Tensor],
-                Aqk: Optional[Tensor], h0: Optional[Tensor], dht: Optional[Tensor], w: Optional[Tensor],
-                qg: Optional[Tensor], kg: Optional[Tensor], v_new: Optional[Tensor], h: Optional[Tensor],
-                cu_seqlens: Optional[Tensor]) -> tuple[Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor]:
-    """(dq, dk, dv, dg, dbeta, db_gate, dw_gate, dh0); outputs a family does not have are empty tensors.
-    Tensors must be contiguous, on one CUDA device, in the dtypes of RewyBwdArgs."""
-    lib = _capi.load()
-    B, T, H, _ = k.shape
-    dev = q.device
-    odt = torch.float32 if out_f32 else torch.bfloat16
-    shape = (B, T, H, 128)
-    vector_gates = family == _capi.GDN2
-    out = dict(
-        dq=torch.empty(shape, dtype=odt, device=dev), dk=torch.empty(shape, dtype=odt, device=dev),
-        dv=torch.empty(shape, dtype=torch.bfloat16, device=dev),
-        dg=torch.empty_like(g) if g is not None else None,
-        dbeta=torch.empty((B, T, H), dtype=torch.float32, device=dev) if not vector_gates else None,
-        db_gate=torch.empty(shape, dtype=odt, device=dev) if vector_gates else None,
-        dw_gate=torch.empty(shape, dtype=odt, device=dev) if vector_gates else None,
-        dh0=torch.empty_like(h0) if h0 is not None else None,   # [B,H,128,128], or [sequences,H,128,128] when packed
-    )
-    a = _capi.BwdArgs()
-    a.family, a.policy, a.B, a.T, a.H = family, policy, B, T, H
-    a.out_dtype = _capi.OUT_F32 if out_f32 else _capi.OUT_BF16
-    a.intra_passes = intra_passes
-    a.state_v_first = int(state_v_first)
-    a.scale = scale
-    if cu_seqlens is not None:   # int32, on the device, [sequences + 1]
-        a.cu_seqlens, a.num_seqs = _capi.ptr(cu_seqlens), cu_seqlens.numel() - 1
-    for name, t in dict(q=q, k=k, v=v, d_o=d_o, Akk=Akk, g=g, beta=beta, b_gate=b_gate, w_gate=w_gate, Aqk=Aqk, h0=h0,
-                        dht=dht, w=w, qg=qg, kg=kg, v_new=v_new, h=h).items():
-        setattr(a, name, _capi.ptr(t))
-    for name, t in out.items():
-        setattr(a, name, _capi.ptr(t))
-    a.workspace = _capi.ptr(workspace)
-    a.workspace_bytes = workspace.numel() * workspace.element_size()
-    fn = getattr(lib, _FAMILY_FN[family])
-    with torch.cuda.device(dev):
-        # Inputs, outputs and workspace are allocated on (or already in use by) the current stream, the same
-        # stream the launches go to, so the caching allocator's stream-ordered reuse keeps them valid.
-        _capi.check(fn(a, _capi.current_stream(dev)), fn.__name__)
-    return tuple(out[n] if out[n] is not None else _empty(dev)
-                 for n in ("dq", "dk", "dv", "dg", "dbeta", "db_gate", "dw_gate", "dh0"))
-
-
-@_family_bwd.register_fake
+@torch.library.register_fake("rewy_b200::family_bwd")
 def _family_bwd_fake(family, policy, out_f32, intra_passes, state_v_first, scale, q, k, v, d_o, Akk, workspace, g, beta, b_gate, w_gate,
                      Aqk, h0, dht, w, qg, kg, v_new, h, cu_seqlens):
     B, T, H, _ = k.shape
@@ -135,7 +92,7 @@ def _c(t, dtype=None):
 def _run(family, policy, B, T, H, scale, tensors, out_dtype, intra_passes, workspace, want_dg, want_dbeta, vector_gates,
          check_status=False, state_v_first=False):
     """tensors: dict name -> tensor or None for every input pointer of RewyBwdArgs."""
-    lib = _capi.load()
+    lib = _capi.load_torch()
     dev = tensors["q"].device
     if out_dtype not in (None, torch.float32, torch.bfloat16):
         raise RuntimeError("rewy_b200 backward: out_dtype must be torch.float32 or torch.bfloat16")
@@ -146,7 +103,7 @@ def _run(family, policy, B, T, H, scale, tensors, out_dtype, intra_passes, works
     elif workspace.numel() * workspace.element_size() < need or workspace.device != dev:
         raise RuntimeError(f"rewy_b200 backward: workspace must hold {need} bytes on {dev}")
     t = tensors
-    r = torch.ops.rewy_b200.family_bwd(
+    r = torch.ops.rewy_b200.family_bwd.default(
         family, policy, out_f32, int(intra_passes or 0), bool(state_v_first), float(scale), t["q"], t["k"], t["v"], t["d_o"], t["Akk"],
         workspace, t["g"], t["beta"], t["b_gate"], t["w_gate"], t["Aqk"], t["h0"], t["dht"], t["w"], t["qg"], t["kg"],
         t["v_new"], t["h"], t.get("cu_seqlens"))

@@ -44,7 +44,7 @@ def chunk_forward(op, q, k, v, g=None, beta=None, b=None, w=None, scale=None, in
     (b [B,T,H,128], w [B,T,H,128]) for 'gdn2'; ``state_v_first``: initial and final state are [B,H,V,K];
     ``check_status`` synchronises and raises if a kernel gave up on a bounded wait; ``cu_seqlens`` (int tensor
     [sequences + 1], lengths multiples of 64, batch of 1): packed sequences, states are [sequences,H,128,128]."""
-    from . import _capi, elementwise
+    from . import _capi, backward, elementwise   # backward defines the operators
     if not q.is_cuda:
         raise RuntimeError("rewy_b200 chunk_forward needs CUDA tensors (there is no CPU fallback); "
                            "chunk_forward_torch is the host restatement used for cross-checks")
@@ -53,7 +53,7 @@ def chunk_forward(op, q, k, v, g=None, beta=None, b=None, w=None, scale=None, in
         raise ValueError("chunk_forward needs BF16 inputs, T % 64 == 0 and K = V = 128")
     scale = K ** -0.5 if scale is None else scale
     dev = q.device
-    lib = _capi.load()
+    lib = _capi.load_torch()
     bf = lambda t: None if t is None else t.to(torch.bfloat16).contiguous()
     q, k, v = bf(q), bf(k), bf(v)
     g_cumsum = None
@@ -69,30 +69,18 @@ def chunk_forward(op, q, k, v, g=None, beta=None, b=None, w=None, scale=None, in
                 g_cumsum = torch.empty(gin.shape, dtype=torch.float32, device=dev)
                 _capi.check(lib.rewy_scalar_gate_cumsum_fwd(_capi.ptr(gin), int(gin.dtype == torch.float32), _capi.ptr(g_cumsum),
                                                             B, T, H, _capi.current_stream(dev)), "rewy_scalar_gate_cumsum_fwd")
-        big = lambda: torch.empty(B, T, H, 128, dtype=torch.bfloat16, device=dev)
-        a64 = lambda: torch.empty(B, T, H, 64, dtype=torch.bfloat16, device=dev)
-        out = dict(o=big(), Aqk=a64(), Akk=a64(), w=big(), u=big(), qg=big(), kg=big(), v_new=big(),
-                   h=torch.empty(B, T // CHUNK, H, 128, 128, dtype=torch.bfloat16, device=dev))
         cu = None if cu_seqlens is None else cu_seqlens.to(device=dev, dtype=torch.int32).contiguous()
         if cu is not None and B != 1:
             raise ValueError("chunk_forward: packed sequences (cu_seqlens) need a batch of 1")
-        nseq = B if cu is None else cu.numel() - 1
-        final = torch.empty(nseq, H, 128, 128, dtype=torch.float32, device=dev) if output_final_state else None
-        ctrl = torch.empty(2, dtype=torch.int32, device=dev)
-        a = _capi.FwdArgs()
-        a.family, a.B, a.T, a.H, a.state_v_first, a.scale = _capi.FAMILY_ID[op], B, T, H, int(bool(state_v_first)), float(scale)
-        keep = [q, k, v, g_cumsum, None if beta is None else beta.float().contiguous(), bf(b), bf(w),
-                None if initial_state is None else initial_state.float().contiguous()]
-        for name, t in zip(("q", "k", "v", "g", "beta", "b_gate", "w_gate", "h0"), keep):
-            setattr(a, name, _capi.ptr(t))
-        for name, t in out.items():
-            setattr(a, name, _capi.ptr(t))
-        a.final_state, a.ctrl = _capi.ptr(final), _capi.ptr(ctrl)
-        if cu is not None:
-            a.cu_seqlens, a.num_seqs = _capi.ptr(cu), nseq
-        _capi.check(lib.rewy_chunk_fwd(a, _capi.current_stream(dev)), "rewy_chunk_fwd")
+        f32 = lambda t: None if t is None else t.float().contiguous()
+        r = torch.ops.rewy_b200.chunk_fwd.default(_capi.FAMILY_ID[op], bool(state_v_first), bool(output_final_state), float(scale),
+                                                  q, k, v, g_cumsum, f32(beta), bf(b), bf(w), f32(initial_state), cu)
+        out = dict(zip(("o", "final_state", "Aqk", "Akk", "w", "u", "qg", "kg", "v_new", "h"), r))
+        if op == "delta":   # without a gate they are the inputs: not written again
+            out["qg"], out["kg"] = q, k
+        final = out["final_state"] if output_final_state else None
         if check_status:
-            _capi.check(lib.rewy_device_status(_capi.ptr(ctrl), _capi.current_stream(dev)), "device status (forward)")
+            _capi.check(lib.rewy_device_status(_capi.ptr(r[-1]), _capi.current_stream(dev)), "device status (forward)")
     out.update(final_state=final, g_cumsum=g_cumsum)
     return out
 

@@ -161,16 +161,28 @@ def operator(op):
         raise ValueError(f"Unknown operator {op!r}")
     optimized = optimized_operator(op)
     signature = inspect.signature(optimized)
+    names = [n for n, p in signature.parameters.items() if p.kind is not p.VAR_KEYWORD]
+    defaults = {n: p.default for n, p in signature.parameters.items() if p.default is not p.empty}
+    required = [n for n in names if n not in defaults]
+
+    def bind(args, kwargs):
+        """Name -> value of every parameter (unknown keywords included); anything unusual goes through ``signature.bind``,
+        which raises as the operator itself would."""
+        given = dict(zip(names, args))
+        if len(args) <= len(names) and not any(n in given for n in kwargs) and all(n in given or n in kwargs for n in required):
+            return {**defaults, **given, **kwargs}
+        bound = signature.bind(*args, **kwargs)
+        bound.apply_defaults()
+        arguments = dict(bound.arguments)
+        arguments.update(arguments.pop("kwargs", {}))
+        return arguments
 
     def call(*args, **kwargs):
         config = _selection.get()
         if config.backend == "original" or op not in config.ops:
             record(op, "original_forward")
             return original_operator(op)(*args, **kwargs)
-        bound = signature.bind(*args, **kwargs)
-        bound.apply_defaults()
-        arguments = dict(bound.arguments)
-        arguments.update(arguments.pop("kwargs", {}))
+        arguments = bind(args, kwargs)
         reason = rejection_reason(op, arguments)
         if reason:
             record(op, "rejected:" + reason)
