@@ -147,7 +147,15 @@ def _pattern(fill, dtype):
     return int.from_bytes(bytes(torch.full((8 // one,), fill, dtype=dtype).view(torch.uint8).tolist()), "little")
 
 
-def _move_rows(fn, tensors, fills, m, T_out):
+def _need_rows(tensors, m, T):
+    """The kernels take the number of rows from the map: a tensor with another one would be read past its end."""
+    for t in tensors:
+        if tuple(t.shape[:2]) != (m.B, T):
+            raise RuntimeError(f"rewy_b200 rows: expected a tensor [{m.B}, {T}, ...], got {list(t.shape)}")
+
+
+def _move_rows(fn, tensors, fills, m, T_in, T_out):
+    _need_rows(tensors, m, T_in)
     _need_cuda(*tensors)
     src = [t.contiguous() for t in tensors]
     out = [torch.empty((t.shape[0], T_out) + tuple(t.shape[2:]), dtype=t.dtype, device=t.device) for t in src]
@@ -162,20 +170,23 @@ def _move_rows(fn, tensors, fills, m, T_out):
 
 def rows_pad(tensors, fills, m, T_padded):
     """[B, T, ...] tensors of any element type -> [B, T_padded, ...], `fills` in the added rows; one launch."""
-    return _move_rows("rewy_rows_pad", tensors, fills, m, T_padded)
+    return _move_rows("rewy_rows_pad", tensors, fills, m, m.T, T_padded)
 
 
 def rows_cut(tensors, m, T):
     """[B, T_padded, ...] -> [B, T, ...]; one launch."""
-    return _move_rows("rewy_rows_cut", tensors, [0] * len(tensors), m, T)
+    return _move_rows("rewy_rows_cut", tensors, [0] * len(tensors), m, m.T_padded, T)
 
 
 def qk_front_fwd(q, k, m, groups, normalize, eps=1e-6):
     """q, k BF16 [B,T,H,128] -> (BF16 [B,T_padded,H*groups,128] twice, rstd FP32 [B,T_padded,H] twice or None): L2
     normalisation, padding rows and the repeat of every head in one pass."""
+    _need_rows((q, k), m, m.T)
     _need_cuda(q, k)
     if q.dtype != torch.bfloat16 or k.dtype != torch.bfloat16 or q.shape[-1] != 128:
         raise RuntimeError("rewy_b200 l2norm: expects BF16 rows of 128 values")
+    if q.shape != k.shape:
+        raise RuntimeError("rewy_b200 q/k front: q and k must have the same shape")
     q, k = _aligned(q), _aligned(k)
     B, _, H, _ = q.shape
     y = [torch.empty(B, m.T_padded, H * groups, 128, dtype=q.dtype, device=q.device) for _ in (q, k)]
@@ -189,6 +200,9 @@ def qk_front_fwd(q, k, m, groups, normalize, eps=1e-6):
 
 def qk_front_bwd(yq, yk, rq, rk, dyq, dyk, m, groups):
     """Backward of qk_front_fwd: dy BF16 or FP32 [B,T_padded,H*groups,128] -> dq, dk BF16 [B,T,H,128]."""
+    _need_rows((yq,), m, m.T_padded)
+    if not yq.shape == yk.shape == dyq.shape == dyk.shape:
+        raise RuntimeError("rewy_b200 q/k front backward: y and dy of q and k must have the same shape")
     _need_cuda(yq, yk, dyq, dyk)
     dyq, dyk = dyq.contiguous(), dyk.contiguous()
     H = yq.shape[2] // groups

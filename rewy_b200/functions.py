@@ -211,6 +211,8 @@ class _Ragged:
         if not self.needed:
             self.total = T
             return
+        if bool((lengths < 0).any()) or int(lengths.sum()) != T:   # the row kernels go by these offsets
+            raise ValueError(f"cu_seqlens must rise and cover the {T} tokens, got {host.tolist()}")
         self.total, self._lengths = int(padded.sum()), lengths
         both = torch.zeros(2, host.numel(), dtype=torch.int32)
         both[0, 1:] = torch.cumsum(lengths, 0)

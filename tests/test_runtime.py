@@ -128,6 +128,29 @@ def test_ragged_lengths_are_padded_to_the_chunk_and_cut_back():
     assert torch.equal(x.grad, torch.full_like(x, 2.0))
 
 
+def test_tensors_with_another_number_of_rows_are_refused_before_any_launch():
+    """The row kernels walk the rows of the map: a beta a row short, a head-first beta, a batch short or offsets that do not
+    cover the tokens must raise (on shapes alone, so before the check for CUDA tensors)."""
+    from rewy_b200 import elementwise as ew
+    from rewy_b200.functions import _Ragged
+    bf = lambda *s: torch.zeros(*s, dtype=torch.bfloat16)
+    for rg, B, T in ((_Ragged(100, "cpu"), 2, 100), (_Ragged(167, "cpu", torch.tensor([0, 37, 101, 167])), 1, 167)):
+        for bad in (bf(B, T - 1, 8), bf(B, T + 1, 8), bf(B, 8, T), bf(B + 1, T, 8), bf(B)):
+            with pytest.raises(RuntimeError, match=r"expected a tensor"):
+                rg.pad_rows(bf(B, T, 8), bad)
+        m = rg.row_map(B)
+        with pytest.raises(RuntimeError, match=r"expected a tensor"):
+            ew.rows_cut([bf(B, T, 8)], m, T)
+        with pytest.raises(RuntimeError, match=r"expected a tensor"):
+            ew.qk_front_fwd(bf(B, T, 2, 128), bf(B, T - 1, 2, 128), m, 1, True)
+        y = bf(B, rg.total, 4, 128)
+        with pytest.raises(RuntimeError, match=r"same shape"):
+            ew.qk_front_bwd(y, y, None, None, y, y[:, :-1], m, 2)
+    for offsets in ([0, 37, 101, 160], [0, 37, 180], [0, 120, 100, 167]):
+        with pytest.raises(ValueError, match="cu_seqlens must rise"):
+            _Ragged(167, "cpu", torch.tensor(offsets))
+
+
 def test_rejection_on_cpu_tensors_is_device():
     from rewy_b200.runtime import rejection_reason
     t = torch.zeros(1, 128, 2, 128, dtype=torch.bfloat16)
