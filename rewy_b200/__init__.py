@@ -24,7 +24,7 @@ def enable(backend="optimized", *, strict=True, ops=None, integrations=()):
     if unknown:
         raise ValueError(f"Unknown integration: {unknown[0]}")
     if backend == "optimized":
-        _capi.load()  # fail here, loudly, if the CUDA library has not been built
+        _capi.load_torch()  # fail here, loudly, if the CUDA library or the torch operators over it have not been built
     if integrations:
         from .integrations import INTEGRATIONS
         for name in integrations:

@@ -159,7 +159,11 @@ def load_torch():
         import torch
         if not TORCH_LIB_PATH.exists():
             raise RuntimeError(f"{TORCH_LIB_PATH} is missing: build it with `python -m rewy_b200.build`")
-        torch.ops.load_library(str(TORCH_LIB_PATH))
+        try:
+            torch.ops.load_library(str(TORCH_LIB_PATH))
+        except OSError as exc:
+            raise RuntimeError(f"{TORCH_LIB_PATH} does not load (built for another torch?), build it again with "
+                               f"`python -m rewy_b200.build`: {exc}") from exc
         _torch_lib_loaded = True
     return lib
 

@@ -30,8 +30,10 @@ _ops.define(   # no gradient formula and no fake implementation: chunk_forward i
     "chunk_fwd(int family, bool state_v_first, bool output_final_state, float scale, Tensor q, Tensor k, Tensor v, Tensor? g, "
     "Tensor? beta, Tensor? b_gate, Tensor? w_gate, Tensor? h0, Tensor? cu_seqlens) -> (Tensor, Tensor, Tensor, Tensor, Tensor, "
     "Tensor, Tensor, Tensor, Tensor, Tensor, Tensor)")
-if _capi.TORCH_LIB_PATH.exists():
+try:   # so that torch.ops.rewy_b200.family_bwd works from here on
     _capi.load_torch()
+except (OSError, RuntimeError):
+    pass   # missing, or built for another torch: enable() and the first call raise it, host-only code does not need it
 
 
 @torch.library.register_fake("rewy_b200::family_bwd")

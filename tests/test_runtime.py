@@ -19,6 +19,37 @@ def test_import_has_no_side_effects():
     assert r.returncode == 0, r.stderr
 
 
+@pytest.mark.parametrize("library", ("missing", "broken"))
+def test_unusable_torch_operators_fail_in_enable_and_not_on_import(tmp_path, library):
+    """Without a loadable rewy_b200_torch.so the host-only modules still import; enable() and the first call raise."""
+    path = tmp_path / "rewy_b200_torch.so"
+    if library == "broken":
+        path.write_bytes(b"not a library")
+    code = f"""
+import pathlib
+from rewy_b200 import _capi
+_capi.TORCH_LIB_PATH = pathlib.Path({str(path)!r})
+import rewy_b200
+from rewy_b200 import backward, functions
+for call in (rewy_b200.enable, _capi.load_torch):
+    try:
+        call()
+    except RuntimeError as e:
+        assert "python -m rewy_b200.build" in str(e), e
+    else:
+        raise SystemExit("did not raise")
+"""
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_enable_loads_the_torch_operators():
+    code = ("import rewy_b200; rewy_b200.enable(); import torch; from rewy_b200 import backward; "
+            "assert torch._C._dispatch_has_kernel_for_dispatch_key('rewy_b200::family_bwd', 'CUDA')")
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
 def test_nested_use_backend_restores_on_exception():
     from rewy_b200 import runtime, use_backend
     assert runtime.selection().backend == "original"
