@@ -18,6 +18,7 @@
 // H=32 336 -> 217 us, GDN B=2 T=4096 H=32 202 -> 148 us, GDN2 B=2 T=2048 H=8 68 -> 41 us.  Unrolled: 251, 150, 45; with
 // 512 threads per CTA: 237, 167, 41 (more instructions per result in the inverse).  Bound by instruction issue of the
 // operand pass and by the inverse's chain (5000 of 16000 cycles of a chunk without a vector gate).
+#include "phase_log.cuh"
 #include "tc05.cuh"
 
 namespace rewy {
@@ -259,6 +260,7 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const uint32_t tlane = tb + ((uint32_t)((warp & 3) * 32) << 16);
   const bool leader = warp == 0 && elect_one();
   uint32_t ph = 0;
+  PhaseLog log;  // what the leader has asked for
   bool alive = true;
   auto wait = [&](int b, int code) {
     if (alive) alive = mbar_wait(&bars[b], ph, p.err, code);  // every barrier in use completes once per chunk
@@ -271,11 +273,13 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   };
   auto load_g = [&](int chunk) {
     const Where w = where(chunk);
+    log.request(LB_G);
     mbar_expect_tx(&bars[LB_G], 32768);
     tma_load_3d(sm + LS::G, &tmG, w.h * 128, w.row0, 0, &bars[LB_G]);
   };
   auto load_qk = [&](int chunk) {
     const Where w = where(chunk);
+    log.request(LB_QK);
     mbar_expect_tx(&bars[LB_QK], 32768);
     for (int pn = 0; pn < 2; pn++) {
       tma_load_2d(sm + LS::QK + pn * 16384, &tmQ, w.h * 128 + 64 * pn, w.row0, &bars[LB_QK]);
@@ -284,6 +288,7 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   };
   auto load_v = [&](int chunk) {
     const Where w = where(chunk);
+    log.request(LB_V);
     mbar_expect_tx(&bars[LB_V], 16384);
     for (int pn = 0; pn < 2; pn++) tma_load_2d(sm + VT + pn * VP, &tmV, w.h * 128 + 64 * pn, w.row0, &bars[LB_V]);
   };
@@ -434,7 +439,10 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
         __syncwarp();
       }
-      if (leader) mma_commit(&bars[LB_D]);
+      if (leader) {
+        log.request(LB_D);
+        mma_commit(&bars[LB_D]);
+      }
       __syncwarp();
     } else {
       // ---- scalar gate / none: exact products on the tiles as they landed --------------------------------------
@@ -446,6 +454,7 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           for (int ks = 0; ks < 8; ks++)
             mma_f16_lo(tb + TM_D, dl(LS::QK + (ks >> 2) * 16384 + (ks & 3) * 32, 16),
                        dl(LS::KT + (ks >> 2) * 16384 + (ks & 3) * 32, 16), ID_D, ks > 0);
+          log.request(LB_D);
           mma_commit(&bars[LB_D]);
         }
         __syncwarp();
@@ -583,6 +592,7 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
         for (int ks = 0; ks < 4; ks++)
           mma_f16_lo(tb + TM_U, dl(LS::AK + ks * 32, 16), dl(VT + ks * 2048, VP), ID_WU, ks > 0);
+        log.request(LB_WU);
         mma_commit(&bars[LB_WU]);
       }
       __syncwarp();
@@ -627,7 +637,8 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   }
   if (leader) {
     if (!alive) {  // gave up: no copy or product may still be under way when the CTA exits
-      for (int b = 0; b < LB_COUNT; b++) mbar_wait_limit(&bars[b], ph, nullptr, 0, DRAIN_NS);
+      for (int b = 0; b < LB_COUNT; b++)
+        if ((log.asked >> b) & 1u) mbar_wait_limit(&bars[b], (log.odd >> b) & 1u, nullptr, 0, DRAIN_NS);
     }
     tma_store_wait_read();
   }

@@ -455,3 +455,52 @@ def test_custom_op_is_registered_with_a_shape_only_implementation():
                                   a64, None, None, big, big, big, big, m(B, T // 64, H, 128, 128), None)
     assert [tuple(x.shape) for x in r] == [(B, T, H, 128)] * 4 + [(0,)] + [(B, T, H, 128)] * 2 + [(0,)]
     assert r[0].dtype == torch.float32 and r[5].dtype == torch.float32
+
+
+def test_phase_log_names_the_last_phase_asked_for(tmp_path):
+    """The drain after a give-up of the forward chunk kernel, on the host: its order of requests is followed up to a wait that
+    runs out, for every wait of three chunks; the log must then name, per barrier, exactly the last phase asked for (its
+    parity is that of the number of earlier ones), whether or not the chunk's other barriers have moved on."""
+    source = tmp_path / "phases.cpp"
+    source.write_text("""
+#include <cstdio>
+#include "phase_log.cuh"
+enum { G, QK, V, D, WU, N };
+static int fails = 0;
+static void walk(bool vec, int give_up_at) {
+  rewy::PhaseLog log;
+  int count[N] = {0}, waits = 0;
+  bool alive = true;
+  auto ask = [&](int b) { log.request(b); count[b]++; };
+  auto wait = [&](int) { if (waits++ == give_up_at) alive = false; };
+  ask(QK);
+  ask(vec ? G : V);
+  for (int c = 0; c < 3 && alive; c++) {
+    const bool next = c < 2;
+    if (vec) wait(G);
+    wait(QK);
+    if (vec || alive) ask(D);
+    wait(D);
+    if (vec && alive) { ask(V); if (next) ask(G); }
+    wait(V);
+    if (alive) ask(WU);
+    wait(WU);
+    if (alive && next) { ask(QK); if (!vec) ask(V); }
+  }
+  for (int b = 0; b < N; b++) {
+    const bool asked = (log.asked >> b) & 1, odd = (log.odd >> b) & 1;
+    if (asked != (count[b] > 0) || (asked && odd != ((count[b] - 1) & 1))) {
+      std::printf("vec %d give-up %d barrier %d\\n", vec, give_up_at, b);
+      fails++;
+    }
+  }
+}
+int main() {
+  for (int at = 0; at <= 15; at++) { walk(true, at); walk(false, at); }
+  return fails != 0;
+}
+""")
+    program = tmp_path / "phases"
+    subprocess.run(["g++", "-std=c++17", "-x", "c++", f"-I{ROOT / 'rewy_b200' / 'csrc'}", str(source), "-o", str(program)], check=True)
+    r = subprocess.run([str(program)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout
