@@ -84,6 +84,11 @@ __device__ __forceinline__ float2 unpack_bf16(uint32_t u) {
   return __bfloat1622float2(p);
 }
 
+// Sum of four products in one fixed order: whichever kernel normalises a row, the bits are the same.
+__device__ __forceinline__ float dot4(const float* a, const float* b) {
+  return fmaf(a[3], b[3], fmaf(a[2], b[2], fmaf(a[1], b[1], __fmul_rn(a[0], b[0]))));
+}
+
 // Copy a [rows x cols] BF16 tile (cols multiple of 8) from global (row pitch g_ld elements) to
 // shared (row pitch s_ld elements) with 16-byte accesses by the whole CTA.
 template <int ROWS, int COLS>

@@ -90,10 +90,16 @@ __global__ void __launch_bounds__(256) rows_kernel(const __grid_constant__ RowIt
   }
 }
 
-__device__ __forceinline__ float half_sum(float x) {  // over the 16 lanes of a half warp
+// sum_i a[i] b[i] over the 16 lanes of a half warp, in the order of the normalisation kernels in wrappers.cu (a whole warp, four
+// channels per lane: lanes 2l and 2l+1 there are the two halves of lane l here, and meet last)
+__device__ __forceinline__ float half_dot(const float (&a)[8], const float (&b)[8]) {
+  float lo = dot4(a, b), hi = dot4(a + 4, b + 4);
 #pragma unroll
-  for (int m = 8; m > 0; m >>= 1) x += __shfl_xor_sync(0xffffffffu, x, m);
-  return x;
+  for (int m = 8; m > 0; m >>= 1) {
+    lo += __shfl_xor_sync(0xffffffffu, lo, m);
+    hi += __shfl_xor_sync(0xffffffffu, hi, m);
+  }
+  return lo + hi;
 }
 __device__ __forceinline__ void unpack8(const uint4& r, float (&x)[8]) {
   const uint32_t u[4] = {r.x, r.y, r.z, r.w};
@@ -141,11 +147,9 @@ __global__ void __launch_bounds__(256) qk_front_fwd_kernel(const FrontParams p, 
 #pragma unroll
     for (int n = 0; n < ITEMS; n++) {
       if (rstd != nullptr) {
-        float x[8], ss = 0.f;
+        float x[8];
         unpack8(u[n], x);
-#pragma unroll
-        for (int j = 0; j < 8; j++) ss = fmaf(x[j], x[j], ss);
-        const float rs = rsqrtf(half_sum(ss) + p.eps);
+        const float rs = rsqrtf(half_dot(x, x) + p.eps);
 #pragma unroll
         for (int j = 0; j < 8; j++) x[j] *= rs;
         u[n] = pack8(x);
@@ -225,13 +229,11 @@ __global__ void __launch_bounds__(256) qk_front_bwd_kernel(const FrontParams p, 
         }
       }
       if (rstd != nullptr) {  // dx = (dy - y <dy, y>) rstd
-        float y[8], s = 0.f;
+        float y[8];
         unpack8(yv[n], y);
+        const float s = half_dot(g, y);
 #pragma unroll
-        for (int j = 0; j < 8; j++) s = fmaf(g[j], y[j], s);
-        s = half_sum(s);
-#pragma unroll
-        for (int j = 0; j < 8; j++) g[j] = (g[j] - y[j] * s) * rs[n];
+        for (int j = 0; j < 8; j++) g[j] = fmaf(-y[j], s, g[j]) * rs[n];
       }
       if (item < total) *reinterpret_cast<uint4*>(p.dx[z] + (size_t)item * 128 + 8 * lane) = pack8(g);
     }

@@ -30,7 +30,8 @@ __device__ __forceinline__ void store4_bf16(bf16* p, const float (&x)[4]) {
   *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]));
 }
 
-// One warp per row of 128 BF16 values; lane l owns columns 4l .. 4l+3.
+// One warp per row of 128 BF16 values; lane l owns columns 4l .. 4l+3.  Both kernels sum in the order of the front kernels in
+// rows.cu (dot4, then the butterfly), so that a row's result does not depend on which of them the call goes through.
 __global__ void __launch_bounds__(256) l2norm_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y,
                                                           float* __restrict__ rstd, long long rows, float eps) {
   const int lane = threadIdx.x & 31;
@@ -38,7 +39,7 @@ __global__ void __launch_bounds__(256) l2norm_fwd_kernel(const bf16* __restrict_
   for (long long r = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += warps) {
     float v[4];
     load4_bf16(x + r * 128 + 4 * lane, v);
-    const float ss = warp_sum(v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3]);
+    const float ss = warp_sum(dot4(v, v));
     const float rs = rsqrtf(ss + eps);
     float o[4] = {v[0] * rs, v[1] * rs, v[2] * rs, v[3] * rs};
     store4_bf16(y + r * 128 + 4 * lane, o);
@@ -61,11 +62,11 @@ __global__ void __launch_bounds__(256) l2norm_bwd_kernel(const bf16* __restrict_
     } else {
       load4_bf16(static_cast<const bf16*>(dy) + r * 128 + 4 * lane, g);
     }
-    const float s = warp_sum(g[0] * yv[0] + g[1] * yv[1] + g[2] * yv[2] + g[3] * yv[3]);
+    const float s = warp_sum(dot4(g, yv));
     const float rs = rstd[r];
     float o[4];
 #pragma unroll
-    for (int i = 0; i < 4; i++) o[i] = (g[i] - yv[i] * s) * rs;
+    for (int i = 0; i < 4; i++) o[i] = fmaf(-yv[i], s, g[i]) * rs;
     store4_bf16(dx + r * 128 + 4 * lane, o);
   }
 }

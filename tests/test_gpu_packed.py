@@ -62,6 +62,26 @@ def test_packed_batch_equals_its_sequences_run_one_at_a_time(op, saved):
         at += T
 
 
+@pytest.mark.parametrize("op", ("kda", "gdn2", "gdn", "delta"))
+def test_normalised_documents_do_not_depend_on_their_neighbours_lengths(op):
+    """A 128-token document alone goes through the plain normalisation kernels, beside one of 100 tokens through the q/k front
+    pass: forward and every gradient are equal to the last bit."""
+    import rewy_b200 as fdr
+    seqs = [make_inputs(op, 1, T, 2, seed=90 + T, device=DEV, gate_scale=0.1, gate="softplus", state=False) for T in (128, 100)]
+
+    def run(tensors, do, **kw):
+        ins = {n: t.detach().clone().requires_grad_() for n, t in tensors.items()}
+        with fdr.use_backend("optimized", ops=(op,)):
+            o, _ = getattr(fdr, NAMES[op])(**ins, use_qk_l2norm_in_kernel=True, **kw)
+        return (o,) + torch.autograd.grad(o, tuple(ins.values()), do)
+
+    both = run({n: torch.cat([s[n] for s in seqs], 1) for n in ARGS[op]}, torch.cat([s["do"] for s in seqs], 1),
+               cu_seqlens=torch.tensor([0, 128, 228], device=DEV))
+    alone = run({n: seqs[0][n] for n in ARGS[op]}, seqs[0]["do"])
+    for n, x, y in zip(("o",) + ARGS[op], both, alone):
+        assert torch.equal(x[:, :128], y), (op, n)
+
+
 @pytest.mark.parametrize("op,saved", [("kda", True), ("gdn2", False), ("gdn", False), ("delta", False)])
 def test_many_packed_pairs_give_what_few_give(op, saved):
     """160 (sequence, head) pairs go to the whole-state scans, the 32 of a single sequence to the scans split by value
