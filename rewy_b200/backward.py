@@ -30,6 +30,7 @@ _ops.define(   # no gradient formula and no fake implementation: chunk_forward i
     "chunk_fwd(int family, bool state_v_first, bool output_final_state, float scale, Tensor q, Tensor k, Tensor v, Tensor? g, "
     "Tensor? beta, Tensor? b_gate, Tensor? w_gate, Tensor? h0, Tensor? cu_seqlens) -> (Tensor, Tensor, Tensor, Tensor, Tensor, "
     "Tensor, Tensor, Tensor, Tensor, Tensor, Tensor)")
+_ops.define("first_order(Tensor[] grads) -> Tensor[]")   # the same tensors, whose differentiation raises
 try:   # so that torch.ops.rewy_b200.family_bwd works from here on
     _capi.load_torch()
 except (OSError, RuntimeError):

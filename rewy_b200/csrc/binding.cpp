@@ -7,6 +7,8 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/autograd_not_implemented_fallback.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/library.h>
 #include <tuple>
 #include "../../include/rewy_b200.h"
@@ -99,6 +101,20 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tenso
   return {o, fin, Aqk, Akk, w, u, qg, kg, v_new, h, ctrl};
 }
 
+// Inside the backward of an autograd function: the gradients it gives, tied to the function's inputs by a node that raises.
+std::vector<Tensor> first_order(at::TensorList grads) {
+  std::vector<Tensor> out(grads.begin(), grads.end());
+  const auto current = torch::autograd::get_current_node();
+  if (current == nullptr) return out;
+  auto edges = current->next_edges();
+  const auto error = std::make_shared<torch::autograd::Error>("derivative for rewy_b200::family_bwd is not implemented", std::move(edges));
+  for (Tensor& t : out) {
+    t = t.detach();
+    torch::autograd::create_gradient_edge(t, error);
+  }
+  return out;
+}
+
 }  // namespace
 
 // (the schemas are defined in rewy_b200/backward.py)
@@ -110,3 +126,4 @@ TORCH_LIBRARY_IMPL(rewy_b200, Autograd, m) {  // differentiating through them ra
   m.impl("family_bwd", torch::autograd::autogradNotImplementedFallback());
   m.impl("chunk_fwd", torch::autograd::autogradNotImplementedFallback());
 }
+TORCH_LIBRARY_IMPL(rewy_b200, CompositeImplicitAutograd, m) { m.impl("first_order", &first_order); }

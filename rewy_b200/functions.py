@@ -22,6 +22,14 @@ def _cumulative_gate(g, A_log=None, dt_bias=None):
     return _ew.gate_cumsum_fwd(g, A_log, dt_bias)
 
 
+def _first_order(grads):
+    """Gradients that come out of the row kernels, which torch does not see: differentiating them again raises, as it does for
+    the family backward (a torch operator without a derivative).  Called inside an autograd function's backward."""
+    if not torch.is_grad_enabled():   # only a backward with create_graph runs with gradients enabled
+        return tuple(grads)
+    return tuple(torch.ops.rewy_b200.first_order.default(list(grads)))
+
+
 def _front(q, k, rows, groups, normalize):
     """q and k as the kernels take them: L2-normalised (optional), padded, each head repeated to its value heads, in one
     pass.  Returns (q, k, q_rstd, k_rstd)."""
@@ -39,7 +47,8 @@ def _front_backward(ctx, q, k, q_rstd, k_rstd, dq, dk):
         return ctx.rows.cut_rows(dq, dk)
     if ctx.groups == 1 and not ctx.rows.needed:
         return _ew.l2norm_bwd(q, q_rstd, dq), _ew.l2norm_bwd(k, k_rstd, dk)
-    return _ew.qk_front_bwd(q, k, q_rstd, k_rstd, dq, dk, ctx.rows.row_map(q.shape[0]), ctx.groups)
+    grads = _ew.qk_front_bwd(q, k, q_rstd, k_rstd, dq, dk, ctx.rows.row_map(q.shape[0]), ctx.groups)
+    return grads if q_rstd is not None else _first_order(grads)   # (the normalisation ends the graph, as its plain kernels do)
 
 
 class ChunkKDAFunction(torch.autograd.Function):
@@ -236,9 +245,9 @@ class _Ragged:
         if not self.needed:
             out = tensors
         elif self.cu is None:
-            out = tuple(t[:, :self.T] for t in tensors)
+            out = _first_order(t[:, :self.T] for t in tensors)
         else:
-            out = _ew.rows_cut(tensors, self.row_map(1), self.T)
+            out = _first_order(_ew.rows_cut(tensors, self.row_map(1), self.T))
         return out[0] if len(out) == 1 else out
 
     # The output of a fixed batch is cut outside the autograd function, as a view that may be written in place like any

@@ -62,3 +62,27 @@ def test_qk_front_equals_its_steps(B, T, lengths, groups, normalize, dy_dtype):
         assert nrmse(rg.cut(g), dx) <= 4e-3
         if groups == 1:
             assert torch.equal(rg.cut(ew.l2norm_bwd(y, r, dy) if normalize else dy.to(torch.bfloat16)), dx)
+
+
+@pytest.mark.parametrize("name,T,lengths,groups", [("chunk_kda", 167, (100, 67), 1), ("chunk_kda", 100, None, 1),
+                                                   ("chunk_gated_delta_rule", 128, None, 2), ("chunk_delta_rule", 167, (100, 67), 2)])
+def test_second_derivatives_raise_through_the_row_kernels(name, T, lengths, groups):
+    """A gradient taken with create_graph cannot be differentiated again: it raises and is never silently a constant."""
+    import rewy_b200 as fdr
+    gen, H = torch.Generator(device=DEV).manual_seed(4), 2
+    rn = lambda *s: torch.randn(*s, generator=gen, device=DEV)
+    xs = dict(q=rn(1, T, H, 128).bfloat16(), k=torch.nn.functional.normalize(rn(1, T, H, 128), dim=-1).bfloat16(),
+              v=rn(1, T, H * groups, 128).bfloat16(), beta=torch.sigmoid(rn(1, T, H * groups)).bfloat16())
+    if name != "chunk_delta_rule":
+        xs["g"] = -0.1 * torch.rand((1, T, H * groups) + ((128,) if name == "chunk_kda" else ()), generator=gen, device=DEV)
+    xs = {n: x.requires_grad_() for n, x in xs.items()}
+    cu = {} if lengths is None else dict(cu_seqlens=torch.tensor([0, lengths[0], T], device=DEV))
+    with fdr.use_backend("optimized"):
+        o, _ = getattr(fdr, name)(**xs, **cu)
+    for loss in (o.float().sum(), o.float().pow(2).sum()):
+        plain = torch.autograd.grad(loss, tuple(xs.values()), retain_graph=True)
+        again = torch.autograd.grad(loss, tuple(xs.values()), create_graph=True)
+        for n, a, b in zip(xs, plain, again):
+            assert torch.equal(a, b), n
+            with pytest.raises(RuntimeError, match="derivative for rewy_b200::family_bwd is not implemented"):
+                torch.autograd.grad(b.float().sum(), tuple(xs.values()), retain_graph=True, allow_unused=True)
