@@ -58,6 +58,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> famil
   }
   a.workspace = workspace.data_ptr();
   a.workspace_bytes = workspace.nbytes();
+  if (!workspace.is_inference()) workspace.unsafeGetTensorImpl()->bump_version();  // written, as the schema says
   const auto st = at::cuda::getCurrentCUDAStream().stream();
   switch (family) {
     case REWY_KDA: check(rewy_kda_bwd(&a, st), "rewy_kda_bwd"); break;

@@ -543,3 +543,14 @@ def test_concurrent_scans_give_the_same_gradients_as_sequential_ones(op):
     for n, t in seq.items():
         if torch.is_tensor(t):
             assert torch.equal(t, par[n]) and torch.equal(t, par2[n]), (op, n)
+
+
+def test_a_workspace_of_the_caller_counts_as_written():
+    """The schema says that the family backward writes its workspace: torch's version counter has to see it."""
+    from rewy_b200 import backward as bw
+    xs = _inputs("delta", T=128, H=2, seed=1, state=False)
+    sv = forward_saved("delta", xs)
+    ws = torch.empty(_capi.workspace_bytes(_capi.DELTA, _capi.RECOMPUTE, 1, 128, 2), dtype=torch.uint8, device=DEV)
+    version = ws._version
+    bw.delta_backward(xs["q"], xs["k"], xs["v"], xs["beta"], sv["Akk"], 128 ** -0.5, None, xs["do"], None, workspace=ws)
+    assert ws._version > version
