@@ -204,7 +204,9 @@ def qk_front_bwd(yq, yk, rq, rk, dyq, dyk, m, groups):
     if not yq.shape == yk.shape == dyq.shape == dyk.shape:
         raise RuntimeError("rewy_b200 q/k front backward: y and dy of q and k must have the same shape")
     _need_cuda(yq, yk, dyq, dyk)
-    dyq, dyk = dyq.contiguous(), dyk.contiguous()
+    dyq, dyk = _aligned(dyq), _aligned(dyk)
+    if rq is not None:   # read with the layout of the forward, which a saved-tensor hook need not give back
+        yq, yk, rq, rk = _aligned(yq), _aligned(yk), rq.contiguous(), rk.contiguous()
     H = yq.shape[2] // groups
     dq, dk = (torch.empty(yq.shape[0], m.T, H, 128, dtype=torch.bfloat16, device=yq.device) for _ in range(2))
     with torch.cuda.device(yq.device):

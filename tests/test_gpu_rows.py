@@ -64,6 +64,26 @@ def test_qk_front_equals_its_steps(B, T, lengths, groups, normalize, dy_dtype):
             assert torch.equal(rg.cut(ew.l2norm_bwd(y, r, dy) if normalize else dy.to(torch.bfloat16)), dx)
 
 
+def test_saved_tensor_hooks_may_change_the_layout():
+    """Hooks that hand every saved tensor back head-first in memory: the gradients are those without hooks."""
+    import rewy_b200 as fdr
+    gen = torch.Generator(device=DEV).manual_seed(5)
+    rn = lambda *s: torch.randn(*s, generator=gen, device=DEV)
+    xs = dict(q=rn(2, 100, 3, 128).bfloat16(), k=rn(2, 100, 3, 128).bfloat16(), v=rn(2, 100, 6, 128).bfloat16(),
+              beta=torch.sigmoid(rn(2, 100, 6)).bfloat16())
+    xs = {n: x.requires_grad_() for n, x in xs.items()}
+    do = rn(2, 100, 6, 128).bfloat16()
+    head_first = lambda t: t.transpose(1, 2).contiguous().transpose(1, 2) if t.ndim >= 3 else t
+
+    def grads(unpack):
+        with fdr.use_backend("optimized"), torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+            o, _ = fdr.chunk_delta_rule(**xs, use_qk_l2norm_in_kernel=True)
+            return torch.autograd.grad(o, tuple(xs.values()), do)
+
+    for n, a, b in zip(xs, grads(lambda t: t), grads(head_first)):
+        assert torch.equal(a, b), n
+
+
 @pytest.mark.parametrize("name,T,lengths,groups", [("chunk_kda", 167, (100, 67), 1), ("chunk_kda", 100, None, 1),
                                                    ("chunk_gated_delta_rule", 128, None, 2), ("chunk_delta_rule", 167, (100, 67), 2)])
 def test_second_derivatives_raise_through_the_row_kernels(name, T, lengths, groups):
