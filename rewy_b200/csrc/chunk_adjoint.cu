@@ -6,8 +6,9 @@
 //   dk = b*(gamma*eb) + yb/gamma;  db = k*(gamma*eb);  dbeta = sum_k db + sum_v v*P
 //   dg = reverse chunk cumsum of  q*dq + k*b*(gamma*eb) - k*(yb/gamma)  (+ chunk-end term on the last row)
 // with Yc = k*zeta, Qc = q*alpha, Ec = b*k*alpha, alpha = exp2(g-c), zeta = 1/alpha and c the per-channel
-// mid-point of the chunk's cumulative gate; chunks whose gate span reaches VECTOR_SPAN_LIMIT (SCALAR_SPAN_LIMIT) log2
-// units take an exact pairwise path instead of the centered products.
+// mid-point of the chunk's cumulative gate; chunks whose gate span reaches VECTOR_SPAN_FREE (SCALAR_SPAN_LIMIT) log2 units,
+// and with them every chunk that chunk_adjoint_tc.cu leaves to this kernel, take an exact pairwise path instead of the
+// centered products.
 //
 // One kernel replaces, for all four families, the reference's residual-WY producer/consumer
 // (src/fast_delta_rule/kernels/kda_residual_tri_beta.py:9-73, kda_residual_local_beta_consumer.py:23-180),
@@ -105,7 +106,7 @@ __device__ __forceinline__ void chunk_body(const ChunkParams& p, const int n, co
         hi = fmaxf(hi, x);
       }
       c = 0.5f * (lo + hi);
-      if (!(hi - lo < VECTOR_SPAN_LIMIT)) atomicOr(sFlag, 1);
+      if (!(hi - lo < VECTOR_SPAN_FREE)) atomicOr(sFlag, 1);
     } else if (GATE == GATE_SCALAR) {
       float lo = INFINITY, hi = -INFINITY;
       for (int r = 0; r < C; r++) {

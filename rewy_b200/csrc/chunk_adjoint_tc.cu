@@ -21,8 +21,13 @@
 //     into registers once; beta rows are double-buffered and fetched under a tensor-core wait;
 //   * dv and dg leave as tiles by bulk stores; per-token sums go through small per-warp arrays, per-channel
 //     sums through spare TMEM columns (no shared-memory atomics).
-// Chunks whose cumulative gate spans VECTOR_SPAN_LIMIT or more log2 units are not processed here: their indices are appended
-// to a list that the warp-MMA kernel (exact pairwise path) works off afterwards.
+// A vector gate whose span in the chunk reaches VECTOR_SPAN_FREE (a far chunk): [dAqk ; dAkk] are scaled by a power of two before
+// the hi/lo split, and the epilogue takes it out again through its per-channel factors, so that other chunks pay for two flags
+// and one product per token: KDA B=8 T=8192 H=32 2080 -> 2105 us, GDN2 B=2 T=32768 H=32 2643 -> 2538 (fewer spills), the far
+// chunks of a KDA layer (B=2 T=4096 H=16, FP32 out) 144 -> 159.  With the scaling as a factor of every output or in a second
+// body of the chunk loop: 2155 .. 2189 and 2111, 152 .. 166 and 190.  Chunks outside the range of the centred factors
+// (common.cuh) are not processed here: their indices are appended to a list that the warp-MMA kernel (exact pairwise path)
+// works off afterwards.
 #include <cstdio>
 #include "tc05.cuh"
 
@@ -89,9 +94,11 @@ struct Smem {
   static constexpr uint32_t DBP = MINMAX;              // float[8][64] sum_v v*P per token, one row per 16 value columns
   static constexpr uint32_t DBW = DBP + 2048;          // float[16 warps][16 tokens] sum_k k*(gamma eb) of the warp's channels
   static constexpr uint32_t DGW = DBW + 1024;          // float[16][16] same for the scalar-gate rows
+  static constexpr uint32_t WMAX = DGW;                // far chunk: uint32[2][16] per warp: largest |k| and |q|, largest |dA|
   static constexpr uint32_t GL = MINMAX + 4096;        // float[128] last-row gate of the chunk per channel
   static constexpr uint32_t BARS = GL + 512;        // 8 mbarriers
   static constexpr uint32_t TMEM = BARS + 128;         // uint32 tmem base (+ flags)
+  static constexpr uint32_t UNSCALE = TMEM + 16;       // float: what takes the scaling of [dAqk ; dAkk] out again
   static constexpr uint32_t TOTAL = TMEM + 64;
 };
 static_assert(Smem::TOTAL + 1024 <= 232448, "shared memory plan exceeds the 227 KB per-CTA limit");
@@ -179,6 +186,9 @@ __device__ __forceinline__ void mma_ts4(uint32_t d, uint32_t a_tmem, uint32_t b,
   for (int ks = 0; ks < 4; ks++) mma_f16_ts(d, a_tmem + ks * 8, b + ((ks * b_step) >> 4), idesc, accumulate || ks > 0);
 }
 
+// 1 / u for a power of two u
+__device__ __forceinline__ float scale_of(float u) { return __uint_as_float((254u << 23) - __float_as_uint(u)); }
+
 // Sum over the warp of x[lane & 15] for each of the 16 per-thread values (16 shuffles); every lane returns the
 // total of value index (lane & 15).
 __device__ __forceinline__ float warp_sum16(float (&x)[16], int lane) {
@@ -251,6 +261,8 @@ chunk_adjoint_tc_kernel(const __grid_constant__ CUtensorMap tmAkk, const __grid_
   float* sDbW = reinterpret_cast<float*>(sm + Smem::DBW);
   float* sDgW = reinterpret_cast<float*>(sm + Smem::DGW);
   float* sGl = reinterpret_cast<float*>(sm + Smem::GL);
+  uint32_t* sWMax = reinterpret_cast<uint32_t*>(sm + Smem::WMAX);
+  volatile float* sUnscale = reinterpret_cast<volatile float*>(sm + Smem::UNSCALE);  // read where used: no register kept
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + Smem::BARS);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + Smem::TMEM);
   const uint32_t sb = smem_u32(sm);
@@ -390,7 +402,7 @@ chunk_adjoint_tc_kernel(const __grid_constant__ CUtensorMap tmAkk, const __grid_
     if (GATE == GATE_VECTOR && wg == NWG - 1) sGl[kch] = g[HALF - 1];
     // (the tiles these values came from are first written again after the barriers below)
     float cen = 0.f;
-    bool wide = false;
+    bool wide = false, far = false;
     if (GATE != GATE_NONE) {
       float lo = INFINITY, hi = -INFINITY;
 #pragma unroll
@@ -409,6 +421,7 @@ chunk_adjoint_tc_kernel(const __grid_constant__ CUtensorMap tmAkk, const __grid_
       }
       if (GATE == GATE_VECTOR) {
         cen = 0.5f * (lo + hi);
+        far = !(hi - lo < VECTOR_SPAN_FREE);
         wide = !(hi - lo < VECTOR_SPAN_LIMIT);
       } else {
         // A scalar gate is the same for every channel, so its pairwise factor 2^(G_i - G_j), i >= j, is applied to the
@@ -423,19 +436,42 @@ chunk_adjoint_tc_kernel(const __grid_constant__ CUtensorMap tmAkk, const __grid_
     }
     // the previous chunk's output tiles must have left shared memory before their regions are written again
     if (leader) tma_store_wait_read();
-    if (__syncthreads_or(wide ? 1 : 0)) {
-      // wide gate span: leave the chunk to the exact pairwise kernel; drain the loads already in flight
-      if (tid == 0) {
-        wait(BAR_A, 101);
-        int idx = atomicAdd(&p.wide_list[0], 1);
-        p.wide_list[1 + idx] = (b * H + h) * NT + n;  // the pairwise kernel's chunk numbering: (batch, head) major
+    far = __syncthreads_or((GATE == GATE_VECTOR ? far : wide) ? 1 : 0) != 0;
+    if (GATE == GATE_VECTOR && tid == 0) *sUnscale = far ? 0.f : 1.f;  // 0: to be determined
+    if (far) {
+      if (GATE == GATE_VECTOR) {  // the range of k and q counts too: 32 bytes of each tile per thread
+        uint32_t m = 0, mq = 0;
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          const uint4 uk = *reinterpret_cast<const uint4*>(sm + Smem::KT + e * 8192 + tid * 16);
+          const uint4 uq = *reinterpret_cast<const uint4*>(sm + Smem::QT + e * 16384 + tid * 16);
+          m = max_abs2(max_abs2(max_abs2(max_abs2(m, uk.x), uk.y), uk.z), uk.w);
+          mq = max_abs2(max_abs2(max_abs2(max_abs2(mq, uq.x), uq.y), uq.z), uq.w);
+        }
+        m = __reduce_max_sync(0xffffffffu, max(m & 0xFFFFu, m >> 16));
+        mq = __reduce_max_sync(0xffffffffu, max(mq & 0xFFFFu, mq >> 16));
+        if (__any_sync(0xffffffffu, wide)) m = 0xFFFFu;  // out of range whatever k is
+        if (lane == 0) sWMax[warp] = m | (mq << 16);
+        __syncthreads();
+        m = sWMax[lane & 15];
+        wide = !centred_range(__reduce_max_sync(0xffffffffu, m & 0xFFFFu)) || !centred_range(__reduce_max_sync(0xffffffffu, m >> 16));
+      } else {
+        wide = true;
       }
-      ph ^= used;
-      fetch_rows(next_chunk, buf ^ 1);
-      buf ^= 1;
-      alive = __syncthreads_and(alive ? 1 : 0) != 0;
-      if (tid == 0 && alive && next_chunk < p.total_chunks) issue_loads(next_chunk, LOAD_G | LOAD_A);
-      continue;
+      if (wide) {
+        // out of the range of the centred factors: leave the chunk to the exact pairwise kernel; drain the loads already in flight
+        if (tid == 0) {
+          wait(BAR_A, 101);
+          int idx = atomicAdd(&p.wide_list[0], 1);
+          p.wide_list[1 + idx] = (b * H + h) * NT + n;  // the pairwise kernel's chunk numbering: (batch, head) major
+        }
+        ph ^= used;
+        fetch_rows(next_chunk, buf ^ 1);
+        buf ^= 1;
+        alive = __syncthreads_and(alive ? 1 : 0) != 0;
+        if (tid == 0 && alive && next_chunk < p.total_chunks) issue_loads(next_chunk, LOAD_G | LOAD_A);
+        continue;
+      }
     }
     if (warp == 0) {
       if (leader) issue_loads(chunk, LOAD_BC);
@@ -474,7 +510,7 @@ chunk_adjoint_tc_kernel(const __grid_constant__ CUtensorMap tmAkk, const __grid_
     used |= 1u << BAR_P;
 
     // ---- operand tile Yc^T of the matrix-intra products (row = channel, 16 token columns per thread) ---------
-    const float ec = GATE == GATE_NONE ? 1.f : ex2(cen);
+    float ec = GATE == GATE_NONE ? 1.f : ex2(cen);
 #pragma unroll
     for (int t8 = 0; t8 < HALF / 8; t8++) {
       float y[8];
@@ -617,14 +653,37 @@ chunk_adjoint_tc_kernel(const __grid_constant__ CUtensorMap tmAkk, const __grid_
     } else if (tid == 0) {
       wait(BAR_C, 6);
     }
+    const bool scaled = GATE == GATE_VECTOR && *sUnscale == 0.f;  // far chunk
     wait(BAR_HD, 4);
     tc_fence_after_sync();
-    if (alive) {
+    {
       const int i = kch & 63;
       const bool lower_incl = kch < C;  // lanes 0..63: dAqk (diagonal kept); lanes 64..127: dAkk (strictly lower)
-      const float mul = lower_incl ? scale : -1.f;
+      float mul = lower_incl ? scale : -1.f;
       const uint32_t thi = lower_incl ? Smem::HHI : Smem::DHI, tlo = lower_incl ? Smem::HLO : Smem::DLO;
-      {
+      if (scaled) {
+        uint32_t m = 0;
+        if (alive) {
+          float x[16];
+          tmem_ld16(tlane + TM_HD + 16 * wg, x);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; j++) {
+            const int col = 16 * wg + j;
+            if (lower_incl ? col <= i : col < i) m = max(m, __float_as_uint(fabsf(mul * x[j])));
+          }
+        }
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (lane == 0) sWMax[TPB / 32 + warp] = m;
+        __syncthreads();
+        m = __reduce_max_sync(0xffffffffu, sWMax[TPB / 32 + (lane & 15)]);
+        // times 2^-e for a largest entry in 2^e .. 2^(e+1), between 2^-25 and 2^25 (al times it must stay a normal number); 1 if
+        // all are zero and around an infinity or NaN
+        const uint32_t e = m == 0u || (m >> 23) >= 255u ? 127u : min(max(m >> 23, 102u), 152u);
+        if (tid == 0) *sUnscale = __uint_as_float(e << 23);
+        mul *= __uint_as_float((254u - e) << 23);
+      }
+      if (alive) {
         float x[16];
         const int col0 = 16 * wg;
         tmem_ld16(tlane + TM_HD + col0, x);
@@ -732,14 +791,26 @@ chunk_adjoint_tc_kernel(const __grid_constant__ CUtensorMap tmAkk, const __grid_
     }
 
     // ---- epilogue, thread = (key channel, token quarter) ------------------------------------------------------
-    // Factored forms: dq = al*(ec*s*x1 + x2), gamma*eb = al*(ec*x3 + x4), yb/gamma = ze*(x6 + en*x5).
+    // Factored forms: dq = al*(ec*s*x1 + x2), gamma*eb = al*(ec*x3 + x4), yb/gamma = ze*(x6 + en*x5).  In a far chunk x2, x4
+    // and x6 are scaled by up = 1 / unscale: ec and en carry it to the other terms, al and ze take it out.
     // Every token quarter lacks the totals of the tokens after it: partial reverse sums are parked in the (dead) Yc
     // tiles and the carry (plus the chunk-end term) is added after the barrier.
     const float gl = GATE == GATE_VECTOR ? sGl[kch] : (GATE == GATE_SCALAR ? sGs[C - 1] : 0.f);
-    const float en = GATE == GATE_NONE ? 1.f : ex2(gl - cen);  // exp2(g_last - g) = zeta * en
+    float en = GATE == GATE_NONE ? 1.f : ex2(gl - cen);  // exp2(g_last - g) = zeta * en
     float* sPark = reinterpret_cast<float*>(sm + Smem::PARK);  // [64 tokens][128 channels]
     const size_t go0 = base128 + (size_t)t0 * ldt + kch;
     fetch_rows(next_chunk, buf ^ 1);
+    float unscale2 = 1.f;
+    if (GATE == GATE_VECTOR) {
+      const float unscale = *sUnscale;
+      if (unscale != 1.f) {
+#pragma unroll
+        for (int j = 0; j < HALF; j++) g[j] *= unscale;
+        ec *= scale_of(unscale);
+        en *= scale_of(unscale);
+        unscale2 = unscale * unscale;  // ze = 1 / al without the scaling
+      }
+    }
     // pass A (needs X1, X2 only): dq, and q*dq parked for the gate row
     wait(BAR_Q, 12);
     tc_fence_after_sync();
@@ -792,7 +863,7 @@ chunk_adjoint_tc_kernel(const __grid_constant__ CUtensorMap tmAkk, const __grid_
           float al = 1.f, ze = 1.f;
           if (GATE != GATE_NONE) {
             al = g[jj];
-            if (GATE == GATE_VECTOR) ze = rcp(al);
+            if (GATE == GATE_VECTOR) ze = rcp(al) * unscale2;
           }
           const float kk = kf(jj);
           const float bb = VB ? bgf(jj) : sBeta[t];

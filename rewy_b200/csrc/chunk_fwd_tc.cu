@@ -11,7 +11,7 @@
 //     leave in 16-byte pieces and E = b k gamma takes the place of k;
 //   * (I + L)^-1 in FP32 by blocks 16 -> 32 -> 64 with all threads: X21 = -X22 (L21 X11);
 //   * w = Akk E and u = Akk Z with Akk stored twice (M=128), so that lanes 0..63 finish w and lanes 64..127 u.
-// A chunk whose gate spans VECTOR_SPAN_LIMIT uses no centred factors: its two matrices are summed pair by pair here.
+// A chunk outside the range of the centred factors (common.cuh) uses none: its two matrices are summed pair by pair here.
 // The loops are kept rolled (two deep): a chunk's code runs once per chunk, and with everything unrolled the warps waited
 // for instructions more than for anything else (1.9 of 10 cycles per issued instruction, more than for memory).
 // Measured, against the warp-MMA kernel before it (three passes over the inputs, inverse by 64 threads): KDA B=1 T=8192
@@ -332,7 +332,7 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
     }
     __syncwarp();
-    bool wide = false;
+    bool wide = false, far = false;
 
     if (VEC) {
       // ---- centre of the gate per channel ---------------------------------------------------------------------
@@ -360,10 +360,27 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           hi = fmaxf(hi, sMM[rg * 256 + 128 + tid]);
         }
         sCen[tid] = 0.5f * (lo + hi);
+        far = !(hi - lo < VECTOR_SPAN_FREE);
         wide = !(hi - lo < VECTOR_SPAN_LIMIT);
       }
-      wide = __syncthreads_or(wide ? 1 : 0) != 0;
+      far = __syncthreads_or(far ? 1 : 0) != 0;
       wait(LB_QK, 42);
+      if (far) {  // the range of q and k counts (common.cuh): thread = half a row of one of them
+        uint32_t* sMax = reinterpret_cast<uint32_t*>(sMM);
+        const unsigned char* row = sm + (krow ? LS::KT : LS::QK) + wg * 16384;
+        uint32_t m = 0;
+#pragma unroll 2
+        for (int c = 0; c < 8; c++) {
+          const uint4 u = *reinterpret_cast<const uint4*>(row + swz(t, c));
+          m = max_abs2(max_abs2(max_abs2(max_abs2(m, u.x), u.y), u.z), u.w);
+        }
+        m = __reduce_max_sync(0xffffffffu, max(m & 0xFFFFu, m >> 16));
+        if (__any_sync(0xffffffffu, wide)) m = 0xFFFFu;  // out of range
+        if (lane == 0) sMax[warp] = m;
+        __syncthreads();
+        const uint32_t mq = max(max(sMax[0], sMax[1]), max(sMax[4], sMax[5])), mk = max(max(sMax[2], sMax[3]), max(sMax[6], sMax[7]));
+        wide = !centred_range(mq) || !centred_range(mk);
+      }
       // ---- operands of the first product ----------------------------------------------------------------------
       if (alive) {
         const float bs = VB ? 0.f : sBeta[t];

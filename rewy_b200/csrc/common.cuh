@@ -15,15 +15,33 @@ enum GateMode { GATE_NONE = 0, GATE_SCALAR = 1, GATE_VECTOR = 2 };
 
 using bf16 = __nv_bfloat16;
 
-// Largest span (max - min over the 64 tokens of a chunk, log2 units) of a per-channel cumulative gate that the centred
-// factors 2^(G - c), 2^(c - G) take: a chunk that reaches it is summed pair by pair on the CUDA cores, some thirty times
-// as slow.  The factors stay inside 2^-100 .. 2^100.  Below 2^-126 an operand's BF16 lo part is lost: that changes a sum
-// by 2^-126 times the other factor, at most 2^-26 of an entry of size 1, while the hi/lo products carry 2^-16; a sum over
-// the kept (causal) entries stays in FP32 range up to 2^27 times an entry of size 1; entries above the diagonal may
-// overflow and are selected away, never multiplied.  A layer with decay rates up to 16 and time steps up to 0.1 averages
-// up to 165 in its fastest channel.  At B=2 T=4096 H=16 with such a gate: a limit of 80 sent 71 % of the chunks to the
-// pairwise sums (3.65 ms of the backward, 0.55 ms of the forward), 160 a few (0.41 ms and 0.10 ms), 200 none.
+// Span (max - min over the 64 tokens of a chunk, log2 units) of a per-channel cumulative gate, and the centred factors
+// 2^(G - c), 2^(c - G), c its mid-point:
+//   below VECTOR_SPAN_FREE  the factors stay inside 2^-40 .. 2^40 and need no care;
+//   below VECTOR_SPAN_LIMIT they reach 2^-100 and 2^100.  A product of such operands is 2^-100 .. 2^100 of the result, so
+//     the backward first scales the chunk's two gradient matrices by a power of two (2^-25 .. 2^25) that brings the largest
+//     entry towards 1.  Measured at a span of 199 without it: dq off by 4.4e-6 down to gradients of 2^-30, by 1.3e-5 at
+//     2^-35 and 2.1e-4 at 2^-40, infinite at 2^40; with it that lies 25 powers further out, so that 2^-55 .. 2^45 (output
+//     gradient times value) is summed as well as a short span.  The forward's kept (causal) sums have their natural size;
+//     entries above the diagonal may overflow and are selected away, never multiplied.  q and k must not add to the
+//     factors: a chunk whose largest |q| or |k| lies outside 2^-20 .. 2^20 goes to the pairwise sums (inside, an operand's
+//     BF16 lo part keeps its place above 2^-133);
+//   from VECTOR_SPAN_LIMIT on the chunk is summed pair by pair on the CUDA cores, some thirty times as slow.
+// A layer with decay rates up to 16 and time steps up to 0.1 averages up to 165 in its fastest channel.  At B=2 T=4096 H=16
+// with such a gate: a limit of 80 sent 71 % of the chunks to the pairwise sums (3.65 ms of the backward, 0.55 ms of the
+// forward), 160 a few (0.41 ms and 0.10 ms), 200 none.
+constexpr float VECTOR_SPAN_FREE = 80.f;
 constexpr float VECTOR_SPAN_LIMIT = 200.f;
+// largest |x| of a chunk's q or k, as the bits of a BF16 (an infinity or NaN is out of range)
+__device__ __forceinline__ bool centred_range(uint32_t bits) {
+  constexpr uint32_t LOW = (127 - 20) << 7, HIGH = (127 + 20) << 7;
+  return bits == 0 || (bits >= LOW && bits < HIGH);
+}
+// larger magnitudes of two pairs of BF16 (m: none negative; a NaN wins)
+__device__ __forceinline__ uint32_t max_abs2(uint32_t m, uint32_t x) {
+  const __nv_bfloat162 r = __hmax2_nan(*reinterpret_cast<const __nv_bfloat162*>(&m), __habs2(*reinterpret_cast<const __nv_bfloat162*>(&x)));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
 // A scalar gate needs no centred factors unless it rises (its pairwise factor is applied to the 64x64 matrices): limit of
 // the chunks that do.
 constexpr float SCALAR_SPAN_LIMIT = 80.f;
