@@ -88,18 +88,24 @@ def test_cuda_forward_value_first_states_and_no_final_state():
     assert none["final_state"] is None and torch.equal(none["o"], plain["o"])
 
 
-@pytest.mark.parametrize("case", ("strong", "mixed"))
+@pytest.mark.parametrize("case", ("strong", "far", "mixed"))
 def test_cuda_forward_wide_gate_spans_take_the_pairwise_path(case):
-    """Cumulative gates spanning 80 log2 units or more per chunk (about 150 everywhere, or far above 200 in a few
-    channels of one chunk next to ordinary chunks): centred factors would leave the FP32 range, the chunk-local kernel
-    sums those chunks pair by pair."""
-    if case == "strong":
-        xs = make_inputs("kda", 1, 192, 2, seed=10, device=DEV, gate_scale=2.0)
-    else:
-        xs = make_inputs("kda", 1, 192, 2, seed=10, device=DEV, gate_scale=0.1)
+    """Cumulative gates spanning 200 log2 units or more per chunk (in every chunk and head, or in a few channels of one chunk
+    next to ordinary chunks): centred factors would leave the FP32 range, the chunk-local kernel sums those chunks pair by
+    pair.  "far": between 80 and 200 everywhere, the widest that keep the centred factors."""
+    scale = dict(strong=4.0, far=2.0, mixed=0.1)[case]
+    xs = make_inputs("kda", 1, 192, 2, seed=10, device=DEV, gate_scale=scale)
+    if case == "mixed":
         xs["g"][:, 64:128, 0, :32] *= 30
-    span = (xs["g"].float().reshape(1, 3, 64, 2, 128).sum(2).abs().max() * 1.4427).item()
-    assert span > 100, span
+    G = xs["g"].float().reshape(1, 3, 64, 2, 128).cumsum(2) * 1.4427
+    span = (G.amax(2) - G.amin(2)).amax(-1)     # [1, chunk, head]: the widest channel
+    if case == "strong":
+        assert bool((span >= 200).all()), span
+    elif case == "far":
+        assert bool(((span > 80) & (span < 200)).all()), span
+    else:
+        assert (span >= 200).sum() == 1 and span[0, 1, 0] >= 200, span
+    span = span.max().item()
     got = chunk_forward("kda", check_status=True, **_kw("kda", xs))
     ref = _oracle("kda", xs)
     errs = {n: nrmse(ref[n].to(got[n].dtype), got[n]) for n in NAMES}

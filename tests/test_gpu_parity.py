@@ -226,7 +226,14 @@ def test_family_backward_bf16_outputs_and_no_states(op):
     _report(_grad_errs(op, ref, out), 3e-3)
 
 
-@pytest.mark.parametrize("case", ["zero_beta", "tiny_beta", "beta_over_one", "strong_gate", "weak_gate", "zero_gate",
+def _tile_spans(saved):
+    """The widest channel's span of the cumulative gate per (chunk, head), log2 units."""
+    G = saved["g_cumsum"].float()
+    G = G.reshape(G.shape[0], -1, 64, *G.shape[2:])
+    return (G.amax(2) - G.amin(2)).amax(-1)
+
+
+@pytest.mark.parametrize("case", ["zero_beta", "tiny_beta", "beta_over_one", "strong_gate", "far_gate", "weak_gate", "zero_gate",
                                   "mixed_tiles", "nonmonotonic_gate", "positive_gate", "dht_only", "h0_only"])
 def test_kda_edge_cases(case):
     """The reference's named KDA acceptance grid (research/operators/gpu_matrix_20261024/run.py:52-78)."""
@@ -243,7 +250,9 @@ def test_kda_edge_cases(case):
     elif case == "beta_over_one":
         xs["beta"] = (xs["beta"].float() * 2).to(torch.bfloat16)
     elif case == "strong_gate":
-        xs["g"] = xs["g"] * 20          # ~ -1.5 nat per step: spans far above 80 log2 units per chunk
+        xs["g"] = xs["g"] * 40          # ~ -3 nat per step: every chunk spans 200 log2 units and more (pairwise)
+    elif case == "far_gate":
+        xs["g"] = xs["g"] * 20          # ~ -1.5 nat per step: every chunk between 80 and 200 (centred, scaled gradients)
     elif case == "weak_gate":
         xs["g"] = xs["g"] / 100
     elif case == "zero_gate":
@@ -255,6 +264,10 @@ def test_kda_edge_cases(case):
     elif case == "positive_gate":
         xs["g"] = -xs["g"] * 0.2
     saved = forward_saved("kda", xs)
+    spans = _tile_spans(saved)
+    wide = dict(strong_gate=spans.numel(), far_gate=0, mixed_tiles=1).get(case)
+    assert wide is None or int((spans >= 200).sum()) == wide, spans
+    assert case != "far_gate" or bool((spans > 80).all()), spans
     ref = oracle_backward("kda", xs, saved)
     out = _family_call("kda", xs, saved, True)
     errs = _grad_errs("kda", ref, out)
@@ -269,8 +282,10 @@ def test_kda_edge_cases(case):
 @pytest.mark.parametrize("op", ("gdn2", "gdn"))
 def test_strong_gate_pairwise_path(op):
     xs = _inputs(op, T=128, H=2, seed=5)
-    xs["g"] = xs["g"] * (25 if op == "gdn2" else 3)
+    xs["g"] = xs["g"] * (50 if op == "gdn2" else 3)
     saved = forward_saved(op, xs)
+    if op == "gdn2":
+        assert bool((_tile_spans(saved) >= 200).all()), _tile_spans(saved)
     ref = oracle_backward(op, xs, saved)
     out = _family_call(op, xs, saved, op == "gdn2")
     errs = _grad_errs(op, ref, out)
