@@ -113,7 +113,7 @@ typedef struct RewyStageBuffers {
   void* dR;     /* bf16 [B,T,H,128]  high part of dR = kg dh + Aqk^T dO */
   void* dR_lo;  /* bf16 [B,T,H,128]  low part: bf16(dR - dR_hi); P = Akk^T (dR + dR_lo) keeps dv, dbeta inside 2e-3 */
   void* ctrl;   /* int32 [2 + B*H*T/64] control block of the chunk stage: [0] device status word, [1] number of
-                   chunks whose gate span was too wide for the centred products, [2..] their indices */
+                   chunks outside the range of the centred products (a wide gate span), [2..] their indices */
 } RewyStageBuffers;
 
 /* Whole-family backward.  Replace, one for one, the functions the reference's autograd backwards call:

@@ -15,9 +15,10 @@
 // The loops are kept rolled (two deep): a chunk's code runs once per chunk, and with everything unrolled the warps waited
 // for instructions more than for anything else (1.9 of 10 cycles per issued instruction, more than for memory).
 // Measured, against the warp-MMA kernel before it (three passes over the inputs, inverse by 64 threads): KDA B=1 T=8192
-// H=32 336 -> 217 us, GDN B=2 T=4096 H=32 202 -> 148 us, GDN2 B=2 T=2048 H=8 68 -> 41 us.  Unrolled: 251, 150, 45; with
-// 512 threads per CTA: 237, 167, 41 (more instructions per result in the inverse).  Bound by instruction issue of the
-// operand pass and by the inverse's chain (5000 of 16000 cycles of a chunk without a vector gate).
+// H=32 336 -> 217 us (222 since the range of q and k is looked at where the gate spans 80), GDN B=2 T=4096 H=32 202 -> 148
+// us, GDN2 B=2 T=2048 H=8 68 -> 41 us.  Unrolled: 251, 150, 45; with 512 threads per CTA: 237, 167, 41 (more instructions
+// per result in the inverse).  Bound by instruction issue of the operand pass and by the inverse's chain (5000 of 16000
+// cycles of a chunk without a vector gate).
 #include "phase_log.cuh"
 #include "tc05.cuh"
 
@@ -240,7 +241,7 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (tid == 0) atomicCAS(p.err, 0, 40);
     return;
   }
-  // thread = (row t of q or k, a quarter of the columns): TMEM lanes 0..63 are rows of q, 64..127 rows of k
+  // thread = (row t of q or k, half of the columns): TMEM lanes 0..63 are rows of q, 64..127 rows of k
   const int t = (warp & 1) * 32 + lane, krow = (warp >> 1) & 1, wg = warp >> 2;
 
   if (tid == 0) {
@@ -616,7 +617,7 @@ chunk_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
     wait(LB_WU, 45);
     tc_fence_after_sync();
-    // ---- w (lanes 0..63) and u (64..127): 32 channels of row t into the dead E / Z tiles ------------------------------
+    // ---- w (lanes 0..63) and u (64..127): 64 channels of row t into the dead E / Z tiles ------------------------------
     if (alive) {
       const int c0 = wg * (128 / NG);
       unsigned char* dst = sm + (krow ? VT + (c0 >> 6) * VP : LS::KT + (c0 >> 6) * 16384);
